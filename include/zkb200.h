@@ -336,8 +336,9 @@ int zkb_msm_fixed_batch(const zkb_msm_job* jobs, int count, void* workspace, siz
  * as a power of two within 8..64, or within 8..16 for zkb_msm and
  * zkb_msm_no_alloc), "msm.call_pairs_cap" (16: that upper limit for the
  * one-MSM calls, 8..64; shorter bucket blocks let work on other streams reach
- * the SMs sooner), "msm.slots_per_thread" (8), "msm.reduce_log_segment" (4: the
- * first reduction level sums 16 buckets a lane, 512 a warp), "msm.sort" (1:
+ * the SMs sooner), "msm.slots_per_thread" (8: runs a quad of lanes adds of a
+ * bucket's merge chunk, 256 a block), "msm.reduce_log_segment" (4: the first
+ * reduction level sums 16 buckets a quad of lanes, 512 a block), "msm.sort" (1:
  * pairs grouped by a counting sort that skips zero digits; 0: a radix sort
  * of all pairs; the same points either way),
  * "ntt.max_log_radix" (log2 of the largest sub-transform one NTT pass does,

@@ -131,3 +131,17 @@ def test_mul_generator_reproduces_the_references_bases(case):
     assert hashlib.sha256(np.ascontiguousarray(bases, dtype="<u8").tobytes()).hexdigest() == case["bases_sha256"]
     x = po.from_mont(wl.rows_to_ints(bases[0:1, 0])[0], P)
     assert x == h(case["bases_first"][0])
+
+
+def test_to_affine_inverts_every_kind_of_z():
+    """The inversion's edges: Z one, small, p - 1, half of p, powers of two, all-ones limbs, random."""
+    import random
+
+    rng = random.Random(41)
+    zs = [1, 2, 3, P - 1, P - 2, P // 2, (P + 1) // 2, 2**64 - 1, 2**128 - 1, 2**253, P - 2**200]
+    zs += [pow(2, e, P) for e in range(0, 512, 7)] + [rng.randrange(1, P) for _ in range(200)]
+    # stored rows hold z 2^256 mod p, so also the z whose rows are those edge values
+    zs += [z * pow(2, -256, P) % P for z in zs]
+    x, y = G.affine()
+    jac = curve_gpu.jacobian_to_device([(x * z * z % P, y * z * z * z % P, z) for z in zs])
+    assert curve_gpu.from_device(jac) == [G] * len(zs)

@@ -351,3 +351,28 @@ def test_reduction_segments_in_batches_and_fixed_base_tables():
         assert got == alone, log_l
         got_t = _with_knobs(knobs, lambda: batch.msm_fixed_batch(table, scs))
         assert got_t == alone, log_l
+
+
+# ------------------------------------------------------------------
+# Merge of the bucket runs (8 pairs a run at these sizes; a bucket of more than 32 runs is
+# summed in chunks of 256, and chunk sums again)
+# ------------------------------------------------------------------
+
+
+@pytest.mark.parametrize("sort", [1, 0])
+@pytest.mark.parametrize("runs", [1, 2, 31, 32, 33, 34, 255, 256, 257, 258, 513, 8300])
+def test_one_bucket_of_many_runs(runs, sort):
+    """One bucket holds every pair but a few: distinct points, and equal ones (whose runs'
+    sums are equal points, so that the merge's additions double)."""
+    n = 8 * runs - 3
+    scalars = np.zeros((n, 4), dtype=np.uint64)
+    scalars[:, 0] = 1
+    scalars[0, 0], scalars[n - 1, 0] = 3, 2  # a bucket on either side
+    k = wl.base_scalars(311, n)
+    bases = curve_gpu.mul_generator(k)
+    ks = wl.rows_to_ints(k)
+    want = G * ((sum(ks) + 2 * ks[0] + ks[n - 1]) % R) if n > 1 else G * (2 * ks[0])
+    same = bases[:1].expand(n, 2, 4).contiguous()
+    knobs = {"msm.sort": sort, "msm.pairs_per_thread": 8}
+    assert _with_knobs(knobs, lambda: msm_pippenger_rows(bases, scalars, window_size=8)) == want
+    assert _with_knobs(knobs, lambda: msm_pippenger_rows(same, scalars, window_size=8)) == G * (ks[0] * (n + 3) % R)

@@ -322,72 +322,6 @@ __device__ __forceinline__ void xyzz_dbl(Xyzz& r, const Xyzz& p) {
   fe_copy(r.y, y3);
 }
 
-// 2P in Jacobian coordinates with the products of M: dbl-2009-l as
-// jac_double (2 products and 5 squarings, against 6 and 3 for xyzz_dbl).
-// For a chain of doublings on one thread (the MSM's final combination).
-template <class M>
-__device__ __forceinline__ void jac_dbl_m(Jac& r, const Jac& p) {
-  G1F f;
-  if (fe_is_zero(p.z) || fe_is_zero(p.y)) {
-    jac_set_identity(r);
-    return;
-  }
-  uint32_t a[8], b[8], c[8], d[8], e[8], t[8], x3[8], y3[8], z3[8];
-  M::sqr(a, p.x);
-  M::sqr(b, p.y);
-  M::sqr(c, b);
-  fe_add(t, p.x, b, f);
-  M::sqr(t, t);
-  fe_sub(t, t, a, f);
-  fe_sub(t, t, c, f);
-  fe_dbl(d, t, f);
-  fe_dbl(e, a, f);
-  fe_add(e, e, a, f);
-  M::sqr(x3, e);
-  fe_dbl(t, d, f);
-  fe_sub(x3, x3, t, f);
-  fe_sub(t, d, x3, f);
-  M::mul(y3, e, t);
-  fe_dbl(t, c, f);
-  fe_dbl(t, t, f);
-  fe_dbl(t, t, f);
-  fe_sub(y3, y3, t, f);
-  M::mul(t, p.y, p.z);
-  fe_dbl(z3, t, f);
-  fe_copy(r.x, x3);
-  fe_copy(r.y, y3);
-  fe_copy(r.z, z3);
-}
-
-// XYZZ (x = X / ZZ, y = Y / ZZZ, ZZ^3 = ZZZ^2) to Jacobian: (X ZZ^2, Y ZZ^3, ZZZ),
-// since (X ZZ^2) / ZZZ^2 = X / ZZ and (Y ZZ^3) / ZZZ^3 = Y / ZZZ. No inversion.
-template <class M>
-__device__ __forceinline__ void xyzz_to_jac(Jac& r, const Xyzz& p) {
-  if (xyzz_is_identity(p)) {
-    jac_set_identity(r);
-    return;
-  }
-  uint32_t zz2[8], zz3[8];
-  M::sqr(zz2, p.zz);
-  M::mul(zz3, zz2, p.zz);
-  M::mul(r.x, p.x, zz2);
-  M::mul(r.y, p.y, zz3);
-  fe_copy(r.z, p.zzz);
-}
-
-// Jacobian to XYZZ: (X, Y, Z^2, Z^3).
-template <class M>
-__device__ __forceinline__ void jac_to_xyzz(Xyzz& r, const Jac& p) {
-  if (fe_is_zero(p.z)) {
-    xyzz_set_identity(r);
-    return;
-  }
-  M::sqr(r.zz, p.z);
-  M::mul(r.zzz, r.zz, p.z);
-  fe_copy(r.x, p.x);
-  fe_copy(r.y, p.y);
-}
-
 // P += (x2, y2), madd-2008-s: P' = x2 ZZ1 - X1, R = y2 ZZZ1 - Y1, PP = P'^2,
 // PPP = P' PP, Q = X1 PP, X3 = R^2 - PPP - 2Q, Y3 = R (Q - X3) - Y1 PPP,
 // ZZ3 = ZZ1 PP, ZZZ3 = ZZZ1 PPP. Special cases: P the identity gives Q;
@@ -476,6 +410,120 @@ __device__ __forceinline__ void xyzz_add(Xyzz& r, const Xyzz& p, const Xyzz& q) 
   fe_copy(r.x, t);
   fe_copy(r.zz, zz);
   fe_copy(r.zzz, zzz);
+}
+
+// ---- XYZZ points spread over four lanes --------------------------------------
+//
+// In a chain of additions on one thread the 14 products of each wait for one
+// another only four deep. A quad of lanes (lane & 3 = 0..3) holds one point, a
+// coordinate per lane (X, Y, ZZ, ZZZ), and runs the formulas' independent
+// products side by side: an addition is four products long instead of 14, a
+// doubling three instead of nine, and a point takes 8 registers of a lane instead
+// of 32. Costs: 16 (12) products are issued for 14 (9) and the values cross lanes
+// by shuffles, so the form is for stages that are bound by latency: the merge of
+// the bucket runs, the bucket reduction, the final combination. Every lane of the
+// warp takes part in each call (a quad with no work adds the identity, all zeros).
+
+__device__ __forceinline__ void shfl8_xor(uint32_t r[8], const uint32_t a[8], int mask) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j) r[j] = __shfl_xor_sync(0xffffffffu, a[j], mask);
+}
+// lane k of each quad to the quad's four lanes
+__device__ __forceinline__ void shfl8_quad(uint32_t r[8], const uint32_t a[8], int k) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j) r[j] = __shfl_sync(0xffffffffu, a[j], k, 4);
+}
+// r = c ? a : b
+__device__ __forceinline__ void sel8(uint32_t r[8], bool c, const uint32_t a[8], const uint32_t b[8]) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j) r[j] = c ? a[j] : b[j];
+}
+
+// a := 2a, dbl-2008-s-1 as xyzz_dbl. The identity (ZZ = 0) and Y = 0 both give
+// ZZ = ZZZ = 0 by the formula itself.
+__device__ __forceinline__ void quad_dbl(uint32_t a[8]) {
+  const G1F f;
+  const int q = threadIdx.x & 3;
+  uint32_t x[8], y[8], s[8], v[8], m[8], t[8], w[8];
+  fe_add(x, a, a, f);
+  sel8(x, q == 1, x, a);   // X, U = 2Y
+  fe_mul(s, x, x, f);      // X^2, V
+  shfl8_quad(v, s, 1);
+  shfl8_quad(w, a, 0);     // X
+  fe_add(m, s, s, f);
+  fe_add(m, m, s, f);      // lane 0: M = 3 X^2
+  sel8(x, q >= 2, a, x);
+  sel8(x, q == 3, w, x);
+  sel8(x, q == 0, m, x);
+  sel8(y, q == 0, m, v);
+  fe_mul(t, x, y, f);      // M^2, W = U V, ZZ3 = ZZ V, S = X V
+  shfl8_xor(s, t, 3);      // lane 0: S
+  shfl8_quad(w, t, 1);     // W
+  fe_sub(v, t, s, f);
+  fe_sub(v, v, s, f);      // lane 0: X3 = M^2 - 2S
+  fe_sub(s, s, v, f);      // lane 0: S - X3
+  sel8(x, q == 0, m, a);
+  sel8(y, q == 0, s, w);
+  fe_mul(y, x, y, f);      // M (S - X3), W Y, -, ZZZ3 = W ZZZ
+  shfl8_xor(x, y, 1);
+  fe_sub(x, x, y, f);      // lane 1: Y3 = M (S - X3) - W Y
+  sel8(a, q == 2, t, y);
+  sel8(a, q == 1, x, a);
+  sel8(a, q == 0, v, a);
+}
+
+// a := a + b, add-2008-s as xyzz_add, with its special cases.
+__device__ __forceinline__ void quad_add(uint32_t a[8], const uint32_t b[8]) {
+  const G1F f;
+  const int lane = threadIdx.x & 31, q = lane & 3, base = lane & 28;
+  // bit base + 2 of each: that point's ZZ is zero
+  const unsigned ida = __ballot_sync(0xffffffffu, fe_is_zero(a)) >> (base + 2);
+  const unsigned idb = __ballot_sync(0xffffffffu, fe_is_zero(b)) >> (base + 2);
+  uint32_t x[8], y[8], z[8], d[8], s[8], w[8], pp[8], t[8];
+  shfl8_xor(x, b, 2);
+  fe_mul(z, a, x, f);      // U1 = X1 ZZ2, S1 = Y1 ZZZ2, U2 = ZZ1 X2, S2 = ZZZ1 Y2
+  shfl8_xor(x, z, 2);
+  fe_sub(d, z, x, f);      // -P, -R, P = U2 - U1, R = S2 - S1
+  const unsigned zero = __ballot_sync(0xffffffffu, fe_is_zero(d)) >> base;
+  sel8(x, q < 2, d, a);
+  sel8(y, q < 2, d, b);
+  fe_mul(s, x, y, f);      // PP, R^2, ZZ1 ZZ2, ZZZ1 ZZZ2
+  shfl8_xor(w, d, 3);      // lane 0: R, lane 1: P
+  shfl8_quad(pp, s, 0);
+  sel8(x, q == 0, z, s);
+  sel8(x, q == 1, w, x);
+  fe_mul(t, x, pp, f);     // Q = U1 PP, PPP = P PP, ZZ3, -
+  fe_sub(x, s, t, f);      // lane 1: R^2 - PPP
+  shfl8_xor(y, x, 1);
+  fe_sub(y, y, t, f);
+  fe_sub(y, y, t, f);      // lane 0: X3 = R^2 - PPP - 2Q
+  fe_sub(x, t, y, f);      // lane 0: Q - X3
+  shfl8_quad(pp, t, 1);    // PPP
+  sel8(d, q == 1, z, s);
+  sel8(d, q == 0, x, d);
+  sel8(pp, q == 0, w, pp);
+  fe_mul(w, d, pp, f);     // R (Q - X3), S1 PPP, -, ZZZ3
+  shfl8_xor(x, w, 1);
+  fe_sub(x, x, w, f);      // lane 1: Y3
+  sel8(w, q == 2, t, w);
+  sel8(w, q == 1, x, w);
+  sel8(w, q == 0, y, w);   // the sum when neither point is the identity and P != 0
+  // P = 0 (bit 2): equal points double, inverse points cancel (ZZ3 = 0 then, but
+  // ZZZ3 and the rest are set to zero too, as every identity here)
+  const bool special = !(ida & 1) && !(idb & 1) && (zero & 4);
+  if (__any_sync(0xffffffffu, special)) {
+    fe_copy(x, a);
+    quad_dbl(x);
+    if (special) {
+      if (zero & 8) {
+        fe_copy(w, x);
+      } else {
+        fe_zero(w);
+      }
+    }
+  }
+  sel8(w, idb & 1, a, w);
+  sel8(a, ida & 1, b, w);
 }
 
 // The MSM's affine bucket lists mark the point at infinity by bit 255 of x,
