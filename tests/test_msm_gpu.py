@@ -376,3 +376,46 @@ def test_one_bucket_of_many_runs(runs, sort):
     knobs = {"msm.sort": sort, "msm.pairs_per_thread": 8}
     assert _with_knobs(knobs, lambda: msm_pippenger_rows(bases, scalars, window_size=8)) == want
     assert _with_knobs(knobs, lambda: msm_pippenger_rows(same, scalars, window_size=8)) == G * (ks[0] * (n + 3) % R)
+
+
+# ------------------------------------------------------------------
+# Bucket runs whose products reduce on the tensor cores (the default) against the ones with
+# every product in place (msm.call_products = 0)
+# ------------------------------------------------------------------
+
+
+@pytest.mark.parametrize("pairs", [8, 13])
+@pytest.mark.parametrize("n", [1, 2, 7, 8, 9, 31, 32, 33, 255, 257, 2048, 4999])
+def test_tensor_core_runs_equal_the_inlined_ones(n, pairs):
+    """Few distinct points and scalars, so that runs meet equal points (doublings), P beside -P
+    (the sum empties and starts again) and buckets of every length; n and the run length leave
+    part-filled runs and warps."""
+    distinct = _bases(5, 331)
+    rng = np.random.default_rng(n)
+    pick = rng.integers(0, 5, size=n)
+    rows = distinct.cpu().numpy()[pick].copy()
+    ys = wl.rows_to_ints(rows[:, 1])
+    flip = rng.random(n) < 0.4
+    for i in np.nonzero(flip)[0]:
+        rows[i, 1] = np.array([((P - ys[i]) >> (64 * j)) & (2**64 - 1) for j in range(4)], dtype=np.uint64)
+    scalars = np.zeros((n, 4), dtype=np.uint64)
+    scalars[:, 0] = rng.integers(0, 4, size=n)
+    full = rng.random(n) < 0.2
+    scalars[full] = wl.uniform_fr(n, int(full.sum()))
+    for w in (4, 8):
+        want = _with_knobs({"msm.call_products": 0, "msm.pairs_per_thread": pairs},
+                           lambda: msm_pippenger_rows(rows, scalars, window_size=w))
+        got = _with_knobs({"msm.pairs_per_thread": pairs}, lambda: msm_pippenger_rows(rows, scalars, window_size=w))
+        assert got == want, w
+    out = co.msm(rows, scalars, 4, threads=4)
+    assert got == (Point.identity() if out[8] else Point(*wl.rows_to_ints(out[:8].reshape(2, 4))))
+
+
+def test_tensor_core_runs_in_a_batch_of_uneven_jobs():
+    from zkgpu import batch
+
+    bases = _bases(3000, 351)
+    scs = [(wl.skewed_scalars if k % 2 else wl.uniform_fr)(360 + k, n) for k, n in enumerate((1, 3000, 17, 999, 2, 2500))]
+    pts = [bases[: s.shape[0]] for s in scs]
+    want = _with_knobs({"msm.call_products": 0}, lambda: batch.msm_batch(pts, scs, window_sizes=[6] * len(scs)))
+    assert batch.msm_batch(pts, scs, window_sizes=[6] * len(scs)) == want

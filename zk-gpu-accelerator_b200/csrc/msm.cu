@@ -43,6 +43,7 @@
 #include "curve.cuh"
 #include "fanout.h"
 #include "field_host.h"
+#include "field_tc.cuh"
 #include "profile.h"
 
 namespace zkb {
@@ -481,6 +482,13 @@ struct RunSink {
   }
 };
 
+__device__ __forceinline__ void prefetch_l2(const void* p) {
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+}
+__device__ __forceinline__ void prefetch_l1(const void* p) {
+  asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
+}
+
 // The points of the job that owns bucket key `key`.
 struct JobPoints {
   const uint64_t* points;
@@ -559,6 +567,130 @@ __global__ void __launch_bounds__(128, 4) k_msm_acc_points_batch(const MsmJobs J
                                                                  uint32_t none, uint64_t* buckets,
                                                                  uint64_t* slots, uint32_t* merge_counts) {
   acc_points<true, M>(J, keys, vals, st, E, E_dev, K, none, buckets, slots, merge_counts);
+}
+
+// Level 1 with the reductions of its products on the tensor cores (field_tc.cuh),
+// which takes whole warps: every lane runs K additions, in step. A lane whose bucket
+// changes writes its run out and starts the next; one whose pairs are used up writes
+// its last run and goes on with values that nobody reads. Coordinates stay in
+// [0, p (1 + 2^-16)), canonical when written. The mixed addition is
+// xyzz_add_affine's, its subtractions folded into the products before them
+// (fold_reduce's d) or left open: with every product operand any 256-bit value,
+// 2p - X1, Q - X3 + 2p and 2p - Y1 need no test. An accumulator with no point yet
+// (`has`), and the rare equal x, are put right after the formula. Expects no entry
+// at infinity, i.e. no affine rounds before it.
+//
+// What bounds it: the integer multiply pipe, about 810 of a warp-addition's cycles
+// per SM, and mma.sync beside it, 160 (the two do not overlap on B200); the rest is
+// latency at 16 warps per SM. The next pair and its row are fetched an addition
+// ahead. Measured on B200 against k_msm_acc_points with its shared products: 2^22
+// points 10.25 to 8.79 ms, 777,777 skewed scalars 546 to 500 us, 2^16 214 to 208 us,
+// 1000 points 42.5 us both. Two lanes per run (five products an addition, five
+// blocks per SM) spilled at 96 registers and took 19 % longer.
+template <bool kBatch>
+__global__ void __launch_bounds__(128, 4) k_msm_acc_points_tc(const MsmJobs J, const uint2* pairs, const uint32_t* E_dev,
+                                                             int K, uint32_t none, uint64_t* buckets,
+                                                             uint64_t* slots, uint32_t* merge_counts) {
+  __shared__ __align__(128) unsigned char scratch[4 * kFoldScratch];
+  const G1F f;
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t == 0) merge_counts[0] = merge_counts[1] = 0;  // k_msm_merge counts from here
+  const int64_t E = *E_dev, start = t * K;
+  if ((t & ~(int64_t)31) * K >= E) return;  // the whole warp
+  FoldWarp fw;
+  fw.init(scratch + (threadIdx.x >> 5) * kFoldScratch, f);
+  pairs += start;
+  const int count = start < E ? (int)(start + K < E ? K : E - start) : 0;
+  uint2 next = count ? pairs[0] : make_uint2(none, 0u);
+  uint32_t cur = next.x;
+  bool first = true, has = false;
+  Xyzz acc;
+  xyzz_set_identity(acc);
+  JobPoints jp = job_points(J, (!kBatch || cur == none) ? 0 : cur);
+  auto row = [&](uint32_t v) {
+    const int64_t idx = (int64_t)(v & 0x7fffffffu);
+    return idx < jp.n ? jp.points + 8 * idx : jp.phi + 8 * (idx - jp.n);
+  };
+  auto flush = [&](bool last) {
+    Xyzz a;
+    xyzz_set_identity(a);
+    if (has) {
+      a = acc;
+      fe_reduce_once(a.x, f);
+      fe_reduce_once(a.y, f);
+      fe_reduce_once(a.zz, f);
+      fe_reduce_once(a.zzz, f);
+    }
+    // the keys beside this thread's range are read again here rather than kept
+    const int64_t s0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * K;
+    const RunSink sink{buckets, slots, (int64_t)blockIdx.x * blockDim.x + threadIdx.x,
+                       first && s0 > 0 ? pairs[-1].x : none,
+                       last && s0 + count < (int64_t)*E_dev ? pairs[count].x : none, none};
+    sink.flush(cur, a, first, last);
+  };
+#pragma unroll 1
+  for (int it = 0; it < K; ++it) {
+    // this pair, and the next one and its row on their way
+    const uint2 pair = next;
+    next = make_uint2(none, 0u);
+    if (it + 1 < count) next = pairs[it + 1];
+    if (pair.x != cur) {
+      flush(it >= count);
+      first = false;
+      has = false;
+      cur = pair.x;
+      if (kBatch && cur != none) jp = job_points(J, cur);
+    }
+    const bool on = cur != none;  // none: this lane's pairs are used up
+    const uint64_t* src = on ? row(pair.y) : nullptr;
+    if (kBatch ? next.x == cur && on : next.x != none) prefetch_l1(row(next.y));
+    const uint32_t v = pair.y;
+    uint32_t pp[8], r[8], t8[8], d[8];
+    {
+      Aff q;
+      if (on) {
+        aff_load_nc(q, src);
+      } else {
+        fe_zero(q.x);
+        fe_zero(q.y);
+      }
+      if (v >> 31) fe_p_minus(q.y, q.y, f);
+      mp_minus<2>(d, acc.x, f);
+      fold_mul(pp, q.x, acc.zz, d, fw, f);   // P' = x2 ZZ1 - X1
+      mp_minus<2>(d, acc.y, f);
+      fold_mul(r, q.y, acc.zzz, d, fw, f);   // R = y2 ZZZ1 - Y1
+    }
+    const bool same_x = is_zero_mod_p(pp, f), same_y = is_zero_mod_p(r, f);
+    uint32_t ppp[8];
+    fold_sqr(t8, pp, nullptr, fw, f);           // PP
+    fold_mul(ppp, pp, t8, nullptr, fw, f);      // PPP
+    fold_mul(acc.zz, acc.zz, t8, nullptr, fw, f);
+    fold_mul(t8, acc.x, t8, nullptr, fw, f);    // Q
+    fold_mul(acc.zzz, acc.zzz, ppp, nullptr, fw, f);
+    mp_minus<4>(d, ppp, f);
+    sub8(d, d, t8);
+    sub8(d, d, t8);                             // 4p - PPP - 2Q
+    fold_sqr(acc.x, r, d, fw, f);               // X3
+    mp_minus<2>(d, acc.x, f);
+    add8(t8, t8, d);                            // Q - X3 + 2p
+    mp_minus<2>(d, acc.y, f);                   // 2p - Y1
+    fold_mul2(acc.y, r, t8, d, ppp, fw, f);     // Y3 = R (Q - X3) - Y1 PPP
+    if (on && (!has || same_x)) {  // src again: L1 has it
+      Aff q;
+      aff_load_nc(q, src);
+      if (v >> 31) fe_neg(q.y, q.y, f);
+      if (!has) {
+        xyzz_from_affine(acc, q);
+        has = true;
+      } else if (same_y) {
+        xyzz_mdbl<InlineMul>(acc, q);
+      } else {
+        has = false;  // P + (-P)
+        xyzz_set_identity(acc);
+      }
+    }
+  }
+  if (cur != none) flush(true);
 }
 
 // ---------------------------------------------------------------------------
@@ -662,9 +794,6 @@ struct AffMeta {
   uint64_t a, b;
 };
 
-__device__ __forceinline__ void prefetch_l2(const void* p) {
-  asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
-}
 
 __device__ __forceinline__ const uint64_t* meta_row(uint64_t v) {
   return reinterpret_cast<const uint64_t*>(v & ~(uint64_t)15);
@@ -1239,7 +1368,7 @@ struct MsmPlan {
   int k1 = 64;     // sorted pairs per bucket thread ("msm.pairs_per_thread", else by size)
   int k2 = 8;      // runs per quad of a merge chunk ("msm.slots_per_thread")
   int log_l = 4;   // log2 of the buckets a quad sums in reduction level 1 ("msm.reduce_log_segment")
-  int call_products = 1;  // bucket kernels call one shared product ("msm.call_products")
+  int call_products = 1;  // 0: bucket kernels expand every product in place ("msm.call_products")
   int counting_sort = 1;  // counting sort (1) or radix sort (0) of the pairs ("msm.sort")
   int table = 0;          // points are fixed-base tables: one bucket set per job
   int64_t windows = 0;    // bucket sets of the batch: count W, or count with tables
@@ -1556,6 +1685,12 @@ static int run_msm(const MsmJobs& J, const MsmPlan& p, char* ws, cudaStream_t s)
       L.pts_n[0] = INT64_MAX;
       auto kern = p.call_products ? k_msm_acc_points<CallMul> : k_msm_acc_points<InlineMul>;
       kern<<<grid, 128, 0, s>>>(L, skeys, svals, st, p.E_list, e_dev, p.k1, p.none, buckets, slots, lists.counts);
+    } else if (p.call_products && p.counting_sort) {
+      // (key, value) words and no points at infinity: the tensor-core form, at least as
+      // fast at every size (k_msm_acc_points_tc)
+      auto kern = p.count > 1 ? k_msm_acc_points_tc<true> : k_msm_acc_points_tc<false>;
+      kern<<<grid, 128, 0, s>>>(J, reinterpret_cast<const uint2*>(skeys), e_dev, p.k1, p.none, buckets, slots,
+                                lists.counts);
     } else if (p.count > 1) {
       auto kern = p.call_products ? k_msm_acc_points_batch<CallMul> : k_msm_acc_points_batch<InlineMul>;
       kern<<<grid, 128, 0, s>>>(J, skeys, svals, st, p.E, e_dev, p.k1, p.none, buckets, slots, lists.counts);
