@@ -10,9 +10,9 @@
 //   2. sort      group the pairs by key, so every bucket's points are
 //                contiguous: either a counting sort ("msm.sort" = 1): the
 //                digits pass counts each key (warp-aggregated atomics, zero
-//                digits skipped), a scan turns counts into bucket offsets, and
-//                a second digits pass scatters each pair into its bucket's
-//                range; or a radix sort of all 2 W n pairs by key (CUB
+//                digits skipped) and numbers its pairs, a scan turns counts into
+//                bucket offsets, and a second digits pass scatters each pair
+//                into its bucket's range; or a radix sort of all 2 W n pairs by key (CUB
 //                onesweep, "msm.sort" = 0), zero digits carrying the largest
 //                key and sorting to the end.
 //   3. buckets   level 1: each thread adds a fixed run of K1 sorted pairs into
@@ -310,76 +310,119 @@ __global__ void __launch_bounds__(256) k_msm_digits(const MsmJobs J, int w, int 
   }
 }
 
-// Counting sort of the pairs (no entry for a zero digit). One thread per scalar,
-// a warp at a time: lanes whose digits fall in the same bucket take one atomic
-// together (__match_any_sync), so a bucket that most scalars share (skewed
-// scalars: digit 1 of window 0) costs one atomic per warp, not per lane.
-// kScatter = false: count[key] += pairs. kScatter = true: each pair takes the
-// next slot of its bucket, cursor[key]++ (the cursors start at the bucket
-// offsets), and is written there as one 8-byte (key, value) word. Within a bucket the order of the pairs
-// varies from run to run; the bucket sum, and so the result, does not.
+// The counting sort's first step: the GLV halves of each scalar, |k1| and |k2| with
+// the sign in bit 127, and (phi != 0) the points phi(P_i) = (beta x_i, y_i) that the k2
+// halves multiply.
+__global__ void __launch_bounds__(256) k_msm_split(const MsmJobs J, uint4* halves, int phi) {
+  FrP fr;
+  FqP f;
+  uint32_t beta[8];
+  glv_beta_mont(beta);
+  const int64_t N = J.first[J.count];
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < N; g += stride) {
+    const int j = job_of_point(J, g);
+    const int64_t i = g - J.first[j];
+    uint32_t sc[8], k1[4], k2[4], neg1, neg2;
+    fe_load_nc(sc, J.scalars[j] + 4 * i);
+    fe_reduce_full(sc, fr, 5);
+    glv_split(sc, k1, neg1, k2, neg2);
+    halves[g] = make_uint4(k1[0], k1[1], k1[2], k1[3] | (neg1 << 31));
+    halves[N + g] = make_uint4(k2[0], k2[1], k2[2], k2[3] | (neg2 << 31));
+    if (phi) {
+      uint32_t x[8], y[8];
+      fe_load_nc(x, J.points[j] + 8 * i);
+      fe_load_nc(y, J.points[j] + 8 * i + 4);
+      fe_mul(x, x, beta, f);
+      fe_store(J.phi[j] + 8 * i, x);
+      fe_store(J.phi[j] + 8 * i + 4, y);
+    }
+  }
+}
+
+// Counting sort of the pairs (no entry for a zero digit). A thread takes one window
+// of both halves of a scalar.
+// Count (kScatter = false): every nonzero digit takes the next number in its bucket
+// (counts[key]++), a warp at a time: lanes whose digits fall in the same bucket take
+// one atomic together (__match_any_sync), so a bucket that most scalars share (skewed
+// scalars: digit 1 of window 0) costs one atomic per warp, not per lane. The number
+// is kept. Scatter: with the counts scanned into bucket offsets, each pair goes to
+// offsets[key] + its number as one 8-byte (key, value) word. The order of a bucket's
+// pairs varies from run to run; the bucket sum, and so the result, does not.
+//
+// The digits of a half are the w-bit fields of |k| + `half` (2^(w-1) in every window
+// but the top one), less 2^(w-1) there, so no borrow runs from window to window and
+// each window is a thread of its own: a small MSM's digits are a few atomics deep
+// instead of 2 W. At large n the atomics bound the count, whose blocks go through the
+// windows together (grid (W, points)) to spread them over all the counters; random
+// 8-byte writes bound the scatter, whose blocks take one window after another (grid
+// (points, W)) so that they stay within one window's pairs, which the L2 cache holds.
+// Measured on B200 against one thread per scalar for all windows with the atomics in
+// both steps, the split and phi kernels included: 1000 points 46 to 15 us, 2^16 59 to
+// 41 us, 2^22 1.72 to 1.49 ms.
 // With a fixed-base table (table = 1) every window shares the job's one set of
 // 2^(w-1) buckets: key = |d| - 1, and the value names the table row of
 // 2^(w win) P (or of its phi image), (point 2 + half) W + win.
 template <bool kScatter>
-__global__ void __launch_bounds__(256) k_msm_bucket_digits(const MsmJobs J, int w, int W, uint32_t none,
-                                                           int table, uint32_t* ctr, uint2* pairs) {
-  FrP fr;
+__global__ void __launch_bounds__(256) k_msm_bucket_digits(const MsmJobs J, const uint4* halves, int w, int W,
+                                                           uint4 half, uint32_t none, int table, uint32_t* counts,
+                                                           const uint32_t* offsets, uint32_t* numbers,
+                                                           uint2* pairs) {
   const int64_t N = J.first[J.count];
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;  // a multiple of 32
-  const int lane = threadIdx.x & 31;
-  const uint32_t half = 1u << (w - 1);
-  for (int64_t g0 = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31); g0 < N; g0 += stride) {
+  const int lane = threadIdx.x & 31, win = kScatter ? blockIdx.y : blockIdx.x;
+  const int64_t block = kScatter ? blockIdx.x : blockIdx.y;
+  const int64_t stride = (int64_t)(kScatter ? gridDim.x : gridDim.y) * blockDim.x;  // a multiple of 32
+  const int32_t top = win + 1 < W ? 1 << (w - 1) : 0;
+  for (int64_t g0 = block * blockDim.x + (threadIdx.x & ~31); g0 < N; g0 += stride) {
     const int64_t g = g0 + lane;  // the whole warp runs every iteration; lanes past N have no digits
-    uint32_t k[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}}, neg[2] = {0, 0};
-    int64_t n = 0, i = 0;
-    uint32_t key_base = 0;
-    if (g < N) {
+    const bool on = g < N;
+    uint32_t key[2] = {none, none}, value[2] = {0, 0}, base[2] = {0, 0};
+    if (on) {
       const int j = job_of_point(J, g);
-      n = J.first[j + 1] - J.first[j];
-      i = g - J.first[j];
-      key_base = (uint32_t)j * J.keys_per_job;
-      uint32_t sc[8];
-      fe_load_nc(sc, J.scalars[j] + 4 * i);
-      fe_reduce_full(sc, fr, 5);
-      glv_split(sc, k[0], neg[0], k[1], neg[1]);
+      const int64_t n = J.first[j + 1] - J.first[j], i = g - J.first[j];
+      const uint32_t key_base = (uint32_t)j * J.keys_per_job;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const uint4 m = halves[h * N + g];
+        uint32_t k[4];
+        asm("add.cc.u32 %0, %4, %8;\n\t"
+            "addc.cc.u32 %1, %5, %9;\n\t"
+            "addc.cc.u32 %2, %6, %10;\n\t"
+            "addc.u32 %3, %7, %11;"
+            : "=r"(k[0]), "=r"(k[1]), "=r"(k[2]), "=r"(k[3])
+            : "r"(m.x), "r"(m.y), "r"(m.z), "r"(m.w & 0x7fffffffu), "r"(half.x), "r"(half.y), "r"(half.z),
+              "r"(half.w));
+        const int32_t d = (int32_t)half_bits(k, win * w, w) - top;
+        const uint32_t mag = (uint32_t)(d < 0 ? -d : d);
+        if (mag) key[h] = key_base + (table ? mag - 1 : (((uint32_t)win << (w - 1)) | (mag - 1)));
+        value[h] = (table ? (uint32_t)((2 * i + h) * W + win) : (uint32_t)(h ? n + i : i)) |
+                   (((m.w >> 31) ^ (d < 0 ? 1u : 0u)) << 31);
+      }
     }
-    for (int h = 0; h < 2; ++h) {
-      const uint32_t point = (uint32_t)(h ? n + i : i);
-      uint32_t carry = 0;
-      for (int win = 0; win < W; ++win) {
-        const uint32_t raw = half_bits(k[h], win * w, w) + carry;
-        uint32_t mag, dneg = 0;
-        if (win + 1 < W && raw > half) {
-          mag = (1u << w) - raw;
-          dneg = 1;
-          carry = 1;
-        } else {
-          mag = raw;
-          carry = 0;
-        }
-        const uint32_t key =
-            mag ? key_base + (table ? mag - 1 : (((uint32_t)win << (w - 1)) | (mag - 1))) : none;
-        const unsigned peers = __match_any_sync(0xffffffffu, key);
-        const int leader = __ffs(peers) - 1;
-        if (!kScatter) {
-          if (lane == leader && key != none) atomicAdd(ctr + key, (uint32_t)__popc(peers));
-        } else {
-          uint32_t base = 0;
-          if (lane == leader && key != none) base = atomicAdd(ctr + key, (uint32_t)__popc(peers));
-          base = __shfl_sync(0xffffffffu, base, leader);
-          if (key != none) {
-            const uint32_t pos = base + (uint32_t)__popc(peers & ((1u << lane) - 1u));
-            const uint32_t row = table ? (uint32_t)((2 * i + h) * W + win) : point;
-            pairs[pos] = make_uint2(key, row | ((neg[h] ^ dneg) << 31));
-          }
-        }
+    uint32_t* num = numbers + (int64_t)win * 2 * N + g;
+    if (!kScatter) {
+      uint32_t peers[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        peers[h] = __match_any_sync(0xffffffffu, key[h]);
+        if (key[h] != none && lane == __ffs(peers[h]) - 1)
+          base[h] = atomicAdd(counts + key[h], (uint32_t)__popc(peers[h]));
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        base[h] = __shfl_sync(0xffffffffu, base[h], __ffs(peers[h]) - 1);
+        if (key[h] != none) num[h * N] = base[h] + (uint32_t)__popc(peers[h] & ((1u << lane) - 1u));
+      }
+    } else {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        if (key[h] != none) pairs[offsets[key[h]] + num[h * N]] = make_uint2(key[h], value[h]);
       }
     }
   }
 }
 
-// phi(P_i) = (beta x_i, y_i), the points that the k2 halves multiply.
+// phi(P_i) = (beta x_i, y_i) alone (the radix sort's form).
 __global__ void __launch_bounds__(256) k_msm_phi(const MsmJobs J) {
   FqP f;
   uint32_t beta[8];
@@ -1186,7 +1229,7 @@ __global__ void __launch_bounds__(128) k_msm_merge_bigs(uint64_t* buckets, const
 }
 
 // ends[b] = the number of sorted keys at most b, b < nbuckets (the radix sort's
-// bucket ends; the counting sort leaves them behind as its cursors).
+// bucket ends; the counting sort has them as its offsets).
 __global__ void __launch_bounds__(256) k_msm_key_ends(const uint32_t* keys, int64_t E, int64_t nbuckets,
                                                       uint32_t* ends) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -1218,8 +1261,8 @@ __global__ void __launch_bounds__(256) k_msm_key_ends(const uint32_t* keys, int6
 // (five more). The chunk's pair is the next level's item; a level with one chunk
 // per window writes the window sums. Latency bounds it (some 30 to 50 dependent
 // additions a level on few warps), hence the quads. Measured on B200 against a
-// point per lane: 1000 points 359 to 133 us, 2^16 512 to 200 us, 2^22 (eight
-// windows of 2^15 buckets) 585 to 377 us.
+// point per lane, 16 items a lane or quad: 1000 points 359 to 133 us, 2^16 512 to
+// 200 us, 2^22 (eight windows of 2^15 buckets) 585 to 377 us.
 //
 // A_in / T_in are [W][G_in] (T_in null at level 1: the buckets are both). Out:
 // [W][chunks_per_window] pairs, or (T_out null) the window sums.
@@ -1367,7 +1410,8 @@ struct MsmPlan {
   int64_t nb = 0;  // buckets per window
   int k1 = 64;     // sorted pairs per bucket thread ("msm.pairs_per_thread", else by size)
   int k2 = 8;      // runs per quad of a merge chunk ("msm.slots_per_thread")
-  int log_l = 4;   // log2 of the buckets a quad sums in reduction level 1 ("msm.reduce_log_segment")
+  int log_l = 4;   // log2 of the most buckets a quad sums in reduction level 1 ("msm.reduce_log_segment")
+  int red_l = 4;   // log2 of the buckets it does sum (first_level_log)
   int call_products = 1;  // 0: bucket kernels expand every product in place ("msm.call_products")
   int counting_sort = 1;  // counting sort (1) or radix sort (0) of the pairs ("msm.sort")
   int table = 0;          // points are fixed-base tables: one bucket set per job
@@ -1394,6 +1438,22 @@ struct MsmPlan {
 static int64_t aff_blocks(int64_t entries, int k) {
   const int64_t per = (int64_t)kAffWorkers * k;
   return std::max<int64_t>(1, std::min<int64_t>((entries + per - 1) / per, 2 * 148));
+}
+
+// log2 of the buckets a quad sums in the first reduction level, at most `cap`. A quad
+// adds its buckets one after another (two additions each), so few of them make a
+// level short, while every block of 32 quads adds some twelve additions of its own:
+// the fewest with about one block an SM (two of them slow each other down as much
+// as the shorter sums gain), and windows of up to 128 buckets in one level. Measured on B200 against
+// 16 a quad, all levels: 1000 points (16 windows of 128 buckets) 133 to 75 us, 2^16
+// (10 of 4096) 200 to 170 us.
+static int first_level_log(int64_t windows, int64_t nb, int cap) {
+  int l = 0;
+  while (l < cap && (windows * nb >> (5 + l)) > 148 * 3 / 2) ++l;
+  if (nb <= 128) {
+    while (l < cap && ((int64_t)32 << l) < nb) ++l;
+  }
+  return l;
 }
 
 // The longest automatic run of sorted pairs a bucket thread takes in a one-MSM
@@ -1460,6 +1520,7 @@ static int make_plan(const int64_t* sizes, int count, int w, MsmPlan& p, int tab
   }
   p.k2 = tune_get("msm.slots_per_thread");
   p.log_l = log_l > 0 ? log_l : tune_get("msm.reduce_log_segment");
+  p.red_l = first_level_log(p.windows, p.nb, p.log_l);
   p.call_products = tune_get("msm.call_products");
   p.T1 = (p.E_list + p.k1 - 1) / p.k1;
   // A bucket of at most 32 runs, or twice the average (uniform scalars), is one
@@ -1509,7 +1570,8 @@ static int make_plan(const int64_t* sizes, int count, int w, MsmPlan& p, int tab
   const int64_t share = p.T1 > 1 ? (2 * p.T1 + p.k2 - 1) / p.k2 : 1;
   p.off_merge_counts = take((size_t)2 * share * 4);
   p.off_merge_sums = take(std::max((size_t)2 * share * 128, (size_t)p.max_chunks * 128));
-  const int64_t red = windows * (p.nb >> p.log_l > 0 ? p.nb >> p.log_l : 1);
+  const int64_t chunks = (p.nb + ((int64_t)32 << p.red_l) - 1) >> (5 + p.red_l);
+  const int64_t red = windows * std::max<int64_t>({p.nb >> p.log_l, chunks, 1});
   p.off_red_s0 = take((size_t)red * 128);
   p.off_red_u0 = take((size_t)red * 128);
   p.off_red_s1 = take((size_t)red * 128);
@@ -1569,41 +1631,48 @@ static int run_msm(const MsmJobs& J, const MsmPlan& p, char* ws, cudaStream_t s)
   int st = 1;
   const uint32_t* e_dev = nullptr;  // pairs written by the counting sort (device)
   const uint64_t* list_pts = nullptr;  // after affine rounds: the points the final list indexes
-  const uint32_t* bucket_ends = reinterpret_cast<const uint32_t*>(ws + p.off_offsets);
+  const uint32_t* bucket_ends = reinterpret_cast<const uint32_t*>(ws + p.off_offsets) + 1;  // counting sort
   if (p.counting_sort) {
     uint32_t* counts = reinterpret_cast<uint32_t*>(ws + p.off_counts);
     uint32_t* offsets = reinterpret_cast<uint32_t*>(ws + p.off_offsets);
+    uint32_t half[4] = {0, 0, 0, 0};  // 2^(w-1) in every window but the top one
+    for (int win = 0; win + 1 < p.W; ++win) {
+      const int bit = win * p.w + p.w - 1;
+      half[bit >> 5] |= 1u << (bit & 31);
+    }
+    const uint4 halves = make_uint4(half[0], half[1], half[2], half[3]);
+    uint4* split = reinterpret_cast<uint4*>(vals1);  // 32 n bytes of 8 W n (W >= 6)
+    const unsigned dblocks = grid_for(p.n, 256);
     {
       ProfSpan span("msm_digits", s);
       ZKB_TRY(check_cuda(cudaMemsetAsync(counts, 0, (size_t)(p.keys_used + 1) * 4, s), "msm count reset"));
-      k_msm_bucket_digits<false><<<grid_for(p.n, 256), 256, 0, s>>>(J, p.w, p.W, p.none, p.table, counts,
-                                                                     nullptr);
+      k_msm_split<<<grid_for(p.n, 256), 256, 0, s>>>(J, split, p.table ? 0 : 1);
+      ZKB_TRY(check_launch("msm scalar split"));
+      k_msm_bucket_digits<false><<<dim3((unsigned)p.W, dblocks), 256, 0, s>>>(J, split, p.w, p.W, halves, p.none, p.table, counts, nullptr,
+                                                       vals0, nullptr);
       ZKB_TRY(check_launch("msm digit count"));
-      if (!p.table) {
-        k_msm_phi<<<grid_for(p.n, 256), 256, 0, s>>>(J);
-        ZKB_TRY(check_launch("msm phi points"));
-      }
     }
     ProfSpan span("msm_sort", s);
     size_t scan_bytes = p.cub_bytes;
     ZKB_TRY(check_cuda(cub::DeviceScan::ExclusiveSum(ws + p.off_cub, scan_bytes, counts, offsets,
                                                      (int)(p.keys_used + 1), s),
                        "msm bucket offsets"));
-    // offsets[keys_used] = the pair count; no key reaches it, so it survives the scatter
-    // the interleaved (key, value) words take the space of keys0 and keys1 (2 x 4 E bytes)
+    // offsets[keys_used] = the pair count
+    // the interleaved (key, value) words take the space of keys0 and keys1 (2 x 4 E bytes), the pairs'
+    // numbers that of vals0
     uint2* pairs = reinterpret_cast<uint2*>(keys0);
-    k_msm_bucket_digits<true><<<grid_for(p.n, 256), 256, 0, s>>>(J, p.w, p.W, p.none, p.table, offsets,
-                                                                  pairs);
+    k_msm_bucket_digits<true><<<dim3(dblocks, (unsigned)p.W), 256, 0, s>>>(J, split, p.w, p.W, halves, p.none, p.table, nullptr, offsets,
+                                                    vals0, pairs);
     ZKB_TRY(check_launch("msm digit scatter"));
     e_dev = offsets + p.keys_used;
     skeys = keys0;
     svals = keys0 + 1;
     st = 2;
     if (p.aff_rounds > 0) {
-      // after the scatter, offsets[b] is the end of bucket b's pairs
+      // offsets[b + 1] is the end of bucket b's pairs
       ProfSpan aspan("msm_affine_rounds", s);
       const int keys = (int)p.keys_used;
-      const uint32_t* in_ends = offsets;
+      const uint32_t* in_ends = offsets + 1;
       const uint64_t* in_pts = nullptr;
       uint32_t* ends[2] = {reinterpret_cast<uint32_t*>(ws + p.off_aff_ends0),
                            reinterpret_cast<uint32_t*>(ws + p.off_aff_ends1)};
@@ -1662,6 +1731,7 @@ static int run_msm(const MsmJobs& J, const MsmPlan& p, char* ws, cudaStream_t s)
     k_msm_key_ends<<<grid_for(p.keys_used, 256), 256, 0, s>>>(skeys, p.E, p.keys_used,
                                                               reinterpret_cast<uint32_t*>(ws + p.off_offsets));
     ZKB_TRY(check_launch("msm bucket ends"));
+    bucket_ends = reinterpret_cast<const uint32_t*>(ws + p.off_offsets);
   }
 
   // 3. buckets
@@ -1725,7 +1795,7 @@ static int run_msm(const MsmJobs& J, const MsmPlan& p, char* ws, cudaStream_t s)
     const uint64_t* A = buckets;
     const uint64_t* T = nullptr;
     int64_t G = p.nb;
-    int lL = p.log_l, r = 0;
+    int lL = p.red_l, r = 0;
     for (;;) {
       const int64_t per = (int64_t)32 << lL;
       const int64_t chunks = (G + per - 1) / per;
