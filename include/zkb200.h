@@ -362,7 +362,10 @@ int zkb_msm_fixed_batch(const zkb_msm_job* jobs, int count, void* workspace, siz
  * with its registers capped for that many blocks per SM), "ntt.lazy" (1:
  * inside a TMA pass, values stay in [0, 2p) between butterfly rounds and are
  * made canonical at the store, for moduli below 2^254; 0: canonical after
- * every operation; the same rows either way);
+ * every operation; the same rows either way), "ntt.matrix" (1: transforms of
+ * 2^20 to 2^24 rows over BN254's Fr run passes of 64 to 256 points as byte matrix
+ * products on the tensor cores, while the knobs of the butterfly passes are at their
+ * defaults; 0: butterfly passes; the same rows either way);
  * "msm.affine_rounds" (rounds in which every bucket's list is halved by affine
  * additions sharing one inversion per block, before the XYZZ levels; 0 = none,
  * the default; -1 = by size; 1..8 forced), "msm.affine_batch" (output entries

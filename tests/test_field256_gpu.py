@@ -435,3 +435,34 @@ def test_tiny_fields_ntt():
         a = list(range(3, 3 + n))
         assert F.to_ints(F.ntt(F.from_ints(a))) == po.ntt(a, p)
         assert F.to_ints(F.ntt(F.from_ints(a), invert=True)) == po.ntt(a, p, invert=True)
+
+
+@pytest.mark.parametrize("table_mb", [4096, 0])
+@pytest.mark.parametrize("log_n", [20, 21, 22, 23])
+def test_matrix_passes_equal_butterfly_passes(log_n, table_mb):
+    """Passes as byte matrix products ("ntt.matrix" = 1) give the butterfly passes' rows for
+    every mix of 64-, 128- and 256-point passes, forward / inverse / coset, with expanded and
+    two-level tables. Inputs include 0, 1, p - 1 and rows of bytes 255 below p, the ends of the
+    byte sums' range; no wait gives up."""
+    from zkgpu import _native
+
+    lib = _native.lib()
+    n = 1 << log_n
+    plain = wl.uniform_fr(500 + log_n, n)
+    plain[:64] = (2**64 - 1, 2**64 - 1, 2**64 - 1, (R >> 192) - 1)
+    plain[64] = (0, 0, 0, 0)
+    plain[n // 2] = _native.limbs(R - 1)
+    plain[n - 1] = (1, 0, 0, 0)
+    rows = _native.torch_module().from_numpy(plain).cuda()  # taken as Montgomery rows
+    try:
+        _native.tune_set("ntt.full_table_mb", table_mb)
+        for invert, coset in ((False, None), (True, None), (False, 5), (True, 7)):
+            _native.tune_set("ntt.matrix", 1)
+            got = BN254_FR.ntt(rows, invert=invert, coset=coset)
+            _native.tune_set("ntt.matrix", 0)
+            want = BN254_FR.ntt(rows, invert=invert, coset=coset)
+            assert bool((got == want).all()), (invert, coset)
+    finally:
+        _native.tune_set("ntt.matrix", 1)
+        _native.tune_set("ntt.full_table_mb", 4096)
+    assert lib.zkb_ntt_wait_timeouts() == 0

@@ -25,6 +25,7 @@
 #include <vector>
 
 #include "field_host.h"
+#include "field_tc.cuh"
 #include "profile.h"
 #include "tma.cuh"
 
@@ -51,6 +52,7 @@ struct RootTables {
   uint64_t* w_fwd = nullptr;
   uint64_t* w_inv = nullptr;
   int log_N = 0, s = 0, log_rmax = 0;
+  unsigned char* mm[2] = {nullptr, nullptr};  // matrix passes' tables, forward and inverse (null: none)
 };
 
 // Per-transform scaling tables: forward coset: g^j = g_lo[j & m] g_hi[j >> gs];
@@ -217,68 +219,6 @@ static std::list<FullEntry> g_fulls;  // most recently used first
 static size_t g_full_bytes = 0;
 static constexpr size_t kMaxFullEntries = 16;
 static constexpr int kMinFullLog = 10;  // below, transforms are one pass with no boundary twiddle
-
-template <class F>
-static int build_roots(const F& f, const TableKey& key, RootTables& t, void** mem,
-                       cudaStream_t s) {
-  t.log_N = key.log_N;
-  t.s = (key.log_N + 1) / 2;
-  t.log_rmax = key.log_N < kMaxLogR ? key.log_N : kMaxLogR;
-  const int64_t n_lo = 1ll << t.s, n_hi = 1ll << (key.log_N - t.s);
-  const int64_t n_w = t.log_rmax > 0 ? (1ll << (t.log_rmax - 1)) : 1;
-  const size_t elems = (size_t)(n_lo + n_hi + 2 * n_w + 4 + 1 /* omega */);
-  uint64_t* base = nullptr;
-  ZKB_TRY(check_cuda(cudaMalloc(&base, elems * 32), "NTT root table allocation"));
-  *mem = base;
-  t.t_lo = base;
-  t.t_hi = t.t_lo + 4 * n_lo;
-  t.w_fwd = t.t_hi + 4 * n_hi;
-  t.w_inv = t.w_fwd + 4 * n_w;
-  uint64_t* bases = t.w_inv + 4 * n_w;
-  uint64_t* omega_dev = bases + 16;
-  ZKB_TRY(check_cuda(cudaMemcpyAsync(omega_dev, key.omega, 32, cudaMemcpyHostToDevice, s),
-                     "NTT root upload"));
-  k_root_bases<<<1, 1, 0, s>>>(f, omega_dev, bases, key.log_N, t.s, t.log_rmax);
-  ZKB_TRY(check_launch("NTT root bases"));
-  k_pow_table<<<grid_for(n_lo, 128), 128, 0, s>>>(f, bases, nullptr, t.t_lo, n_lo);
-  ZKB_TRY(check_launch("NTT root table (low powers)"));
-  k_pow_table<<<grid_for(n_hi, 128), 128, 0, s>>>(f, bases + 4, nullptr, t.t_hi, n_hi);
-  ZKB_TRY(check_launch("NTT root table (high powers)"));
-  k_pow_table<<<grid_for(n_w, 128), 128, 0, s>>>(f, bases + 8, nullptr, t.w_fwd, n_w);
-  ZKB_TRY(check_launch("NTT stage table"));
-  k_pow_table<<<grid_for(n_w, 128), 128, 0, s>>>(f, bases + 12, nullptr, t.w_inv, n_w);
-  ZKB_TRY(check_launch("NTT inverse stage table"));
-  // Other streams may use the entry as soon as it is published.
-  return check_cuda(cudaStreamSynchronize(s), "NTT root table build");
-}
-
-template <class F>
-static int build_scale(const F& f, const ScaleKey& key, int log_n, ScaleTables& t, void** mem,
-                       cudaStream_t s) {
-  t.gs = (log_n + 1) / 2;
-  const int64_t n_lo = 1ll << t.gs, n_hi = 1ll << (log_n - t.gs);
-  const bool tables = key.has_coset != 0;
-  const size_t elems = (size_t)((tables ? n_lo + n_hi : 0) + 4 + 1);
-  uint64_t* base = nullptr;
-  ZKB_TRY(check_cuda(cudaMalloc(&base, elems * 32), "NTT scale table allocation"));
-  *mem = base;
-  uint64_t* bases = base + (tables ? 4 * (n_lo + n_hi) : 0);
-  uint64_t* g_dev = bases + 16;
-  t.scale = bases + 8;
-  ZKB_TRY(check_cuda(cudaMemcpyAsync(g_dev, key.g, 32, cudaMemcpyHostToDevice, s),
-                     "NTT coset upload"));
-  k_scale_bases<<<1, 1, 0, s>>>(f, g_dev, key.has_coset, key.inverse, key.n, t.gs, bases);
-  ZKB_TRY(check_launch("NTT scale bases"));
-  if (tables) {
-    t.g_lo = base;
-    t.g_hi = base + 4 * n_lo;
-    k_pow_table<<<grid_for(n_lo, 128), 128, 0, s>>>(f, bases, nullptr, t.g_lo, n_lo);
-    ZKB_TRY(check_launch("NTT coset table (low powers)"));
-    k_pow_table<<<grid_for(n_hi, 128), 128, 0, s>>>(f, bases + 4, bases + 12, t.g_hi, n_hi);
-    ZKB_TRY(check_launch("NTT coset table (high powers)"));
-  }
-  return check_cuda(cudaStreamSynchronize(s), "NTT scale table build");
-}
 
 // ---------------------------------------------------------------------------
 // The pass kernel
@@ -457,6 +397,16 @@ struct LazyOk<FrP> {
 };
 template <>
 struct LazyOk<FqP> {
+  static constexpr bool value = true;
+};
+
+// The field whose transforms have matrix passes (ntt_matrix.cuh).
+template <class F>
+struct MatrixOk {
+  static constexpr bool value = false;
+};
+template <>
+struct MatrixOk<FrP> {
   static constexpr bool value = true;
 };
 
@@ -1022,6 +972,12 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_ntt_pass_tma(F f, cons
   }
 }
 
+}  // namespace zkb
+
+#include "ntt_matrix.cuh"
+
+namespace zkb {
+
 // ---------------------------------------------------------------------------
 // Batched form: one persistent launch for many transforms
 // ---------------------------------------------------------------------------
@@ -1103,6 +1059,74 @@ __global__ void __launch_bounds__(kBatchThreads) k_ntt_batch(F f, const __grid_c
 // ---------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------
+
+template <class F>
+static int build_roots(const F& f, const TableKey& key, RootTables& t, void** mem,
+                       cudaStream_t s) {
+  t.log_N = key.log_N;
+  t.s = (key.log_N + 1) / 2;
+  t.log_rmax = key.log_N < kMaxLogR ? key.log_N : kMaxLogR;
+  const int64_t n_lo = 1ll << t.s, n_hi = 1ll << (key.log_N - t.s);
+  const int64_t n_w = t.log_rmax > 0 ? (1ll << (t.log_rmax - 1)) : 1;
+  const size_t elems = (size_t)(n_lo + n_hi + 2 * n_w + 4 + 1 /* omega */);
+  const bool mm = MatrixOk<F>::value && t.log_rmax == kMaxLogR;
+  uint64_t* base = nullptr;
+  ZKB_TRY(check_cuda(cudaMalloc(&base, elems * 32 + (mm ? 2 * kMmDirBytes : 0)), "NTT root table allocation"));
+  *mem = base;
+  t.t_lo = base;
+  t.t_hi = t.t_lo + 4 * n_lo;
+  t.w_fwd = t.t_hi + 4 * n_hi;
+  t.w_inv = t.w_fwd + 4 * n_w;
+  uint64_t* bases = t.w_inv + 4 * n_w;
+  uint64_t* omega_dev = bases + 16;
+  ZKB_TRY(check_cuda(cudaMemcpyAsync(omega_dev, key.omega, 32, cudaMemcpyHostToDevice, s),
+                     "NTT root upload"));
+  k_root_bases<<<1, 1, 0, s>>>(f, omega_dev, bases, key.log_N, t.s, t.log_rmax);
+  ZKB_TRY(check_launch("NTT root bases"));
+  k_pow_table<<<grid_for(n_lo, 128), 128, 0, s>>>(f, bases, nullptr, t.t_lo, n_lo);
+  ZKB_TRY(check_launch("NTT root table (low powers)"));
+  k_pow_table<<<grid_for(n_hi, 128), 128, 0, s>>>(f, bases + 4, nullptr, t.t_hi, n_hi);
+  ZKB_TRY(check_launch("NTT root table (high powers)"));
+  k_pow_table<<<grid_for(n_w, 128), 128, 0, s>>>(f, bases + 8, nullptr, t.w_fwd, n_w);
+  ZKB_TRY(check_launch("NTT stage table"));
+  k_pow_table<<<grid_for(n_w, 128), 128, 0, s>>>(f, bases + 12, nullptr, t.w_inv, n_w);
+  ZKB_TRY(check_launch("NTT inverse stage table"));
+  for (int dir = 0; mm && dir < 2; ++dir) {
+    t.mm[dir] = reinterpret_cast<unsigned char*>(base) + elems * 32 + dir * kMmDirBytes;
+    k_mm_tables<<<(4096 + kMmTwiddleRows + 127) / 128, 128, 0, s>>>(f, dir ? t.w_inv : t.w_fwd, t.mm[dir]);
+    ZKB_TRY(check_launch("NTT matrix tables"));
+  }
+  // Other streams may use the entry as soon as it is published.
+  return check_cuda(cudaStreamSynchronize(s), "NTT root table build");
+}
+
+template <class F>
+static int build_scale(const F& f, const ScaleKey& key, int log_n, ScaleTables& t, void** mem,
+                       cudaStream_t s) {
+  t.gs = (log_n + 1) / 2;
+  const int64_t n_lo = 1ll << t.gs, n_hi = 1ll << (log_n - t.gs);
+  const bool tables = key.has_coset != 0;
+  const size_t elems = (size_t)((tables ? n_lo + n_hi : 0) + 4 + 1);
+  uint64_t* base = nullptr;
+  ZKB_TRY(check_cuda(cudaMalloc(&base, elems * 32), "NTT scale table allocation"));
+  *mem = base;
+  uint64_t* bases = base + (tables ? 4 * (n_lo + n_hi) : 0);
+  uint64_t* g_dev = bases + 16;
+  t.scale = bases + 8;
+  ZKB_TRY(check_cuda(cudaMemcpyAsync(g_dev, key.g, 32, cudaMemcpyHostToDevice, s),
+                     "NTT coset upload"));
+  k_scale_bases<<<1, 1, 0, s>>>(f, g_dev, key.has_coset, key.inverse, key.n, t.gs, bases);
+  ZKB_TRY(check_launch("NTT scale bases"));
+  if (tables) {
+    t.g_lo = base;
+    t.g_hi = base + 4 * n_lo;
+    k_pow_table<<<grid_for(n_lo, 128), 128, 0, s>>>(f, bases, nullptr, t.g_lo, n_lo);
+    ZKB_TRY(check_launch("NTT coset table (low powers)"));
+    k_pow_table<<<grid_for(n_hi, 128), 128, 0, s>>>(f, bases + 4, bases + 12, t.g_hi, n_hi);
+    ZKB_TRY(check_launch("NTT coset table (high powers)"));
+  }
+  return check_cuda(cudaStreamSynchronize(s), "NTT scale table build");
+}
 
 static int ilog2(int64_t n) {
   int l = 0;
@@ -1491,6 +1515,56 @@ static int launch_pass_tma(const F& f, const PassLaunch& L, int64_t n, int P, in
   return check_launch("NTT pass launch (TMA)");
 }
 
+// Whether a transform's passes go through k_ntt_pass_mm ("ntt.matrix", default 1):
+// BN254 Fr with the library's tables, every pass of 64, 128 or 256 points on whole
+// 2048-row tiles, at least two tiles for each SM (the blocks are persistent and load
+// 128 KiB of matrices first), and none of the butterfly passes' own knobs set.
+// Measured on B200, butterfly against matrix passes: 2^20 rows 0.250 / 0.237 ms, 2^22
+// 0.916 / 0.722; 2^19 rows are 256 tiles for 148 SMs, two rounds of which the second
+// is three quarters full.
+static bool matrix_passes(const RootTables& rt, const std::vector<PassLaunch>& passes, int64_t n, int sms) {
+  if (!rt.mm[0] || tune_get("ntt.matrix") == 0 || (n >> kMmTileLog) < 2 * sms) return false;
+  if (tune_get("ntt.tma_grid") != 1 || tune_get("ntt.tma_blocks_per_sm") != 0 || tune_get("ntt.lazy") == 0 ||
+      tune_get("ntt.cta_log_elems") != 0 || tune_get("ntt.threads") != 0) {
+    return false;
+  }
+  for (const PassLaunch& L : passes) {
+    const int lc = kMmTileLog - L.a.lr;
+    if (L.a.lr < kMmMinLr || L.a.lr > kMmMaxLr || lc > (L.a.last ? L.a.lR1 : L.a.ls)) return false;
+  }
+  return true;
+}
+
+// One pass through k_ntt_pass_mm: its tensor map (a box is C columns of all R rows,
+// one of the two 16-byte halves) and one block per SM.
+static int launch_pass_mm(const FrP& f, const PassLaunch& L, const RootTables& rt, int64_t n, int sms, cudaStream_t s) {
+  NttPass a = L.a;
+  a.lc = kMmTileLog - a.lr;
+  const uint64_t R = 1ull << a.lr, C = 1ull << a.lc;
+  CUtensorMap map;
+  if (!a.last) {
+    const uint64_t S = 1ull << a.ls, B = R << a.ls;
+    const uint64_t dims[4] = {4, S, R, (uint64_t)n / B};
+    const uint64_t strides[3] = {32, S * 32, B * 32};
+    const uint32_t box[4] = {2, (uint32_t)C, (uint32_t)R, 1};
+    ZKB_TRY(encode_tensor_map_u64(&map, a.in, 4, dims, strides, box));
+  } else {
+    const uint64_t R1 = 1ull << a.lR1, R2 = 1ull << a.lR2;
+    const uint64_t dims[4] = {4, R1, R, R2};
+    const uint64_t strides[3] = {R2 * R * 32, 32, R * 32};
+    const uint32_t box[4] = {2, (uint32_t)C, (uint32_t)R, 1};
+    ZKB_TRY(encode_tensor_map_u64(&map, a.in, 4, dims, strides, box));
+  }
+  constexpr uint32_t mu = FoldTable<FrP>().mu;
+  const MmPass mp{n >> kMmTileLog, rt.mm[a.inverse], mu};
+  const size_t smem = 2 * (size_t)kMmPlane + kMmMatrixBytes + ((size_t)32 << a.lr) + 1024;
+  ZKB_TRY(check_cuda(cudaFuncSetAttribute(k_ntt_pass_mm<FrP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+                     "NTT matrix pass shared memory attribute"));
+  ProfSpan span(a.last ? "ntt_last_pass" : "ntt_column_pass", s);
+  k_ntt_pass_mm<FrP><<<(unsigned)std::min<int64_t>(mp.ntiles, sms), kMmThreads, smem, s>>>(f, a, mp, map);
+  return check_launch("NTT pass launch (matrix)");
+}
+
 template <class F>
 static int run_ntt(const F& f, const zkb_field* field, const uint64_t* in, uint64_t* out,
                    int64_t n, int invert, const uint64_t* omega, const uint64_t* coset,
@@ -1516,11 +1590,18 @@ static int run_ntt(const F& f, const zkb_field* field, const uint64_t* in, uint6
   const bool tma = P >= 2 && tune_get("ntt.tma") != 0;
   int sms = 0;
   if (tma) ZKB_TRY(sm_count(device, &sms));
+  const bool matrix = tma && matrix_passes(rt, passes, n, sms);
   for (int q = 0; q < P; ++q) {
     if (!passes[q].a.last) {
       ZKB_TRY(lookup_twiddles(f, key, rt, passes[q].a.lr, passes[q].a.ls, invert, &passes[q].a.t_full, s));
     }
     const PassLaunch& L = passes[q];
+    if constexpr (MatrixOk<F>::value) {
+      if (matrix) {
+        ZKB_TRY(launch_pass_mm(f, L, rt, n, sms, s));
+        continue;
+      }
+    }
     if (tma) {
       ZKB_TRY(launch_pass_tma(f, L, n, P, sms, s, q));
       continue;
