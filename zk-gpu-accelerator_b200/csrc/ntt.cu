@@ -62,7 +62,11 @@ struct ScaleTables {
   uint64_t* g_hi = nullptr;
   uint64_t* scale = nullptr;  // one element: n^-1 (Montgomery)
   uint64_t* g_full = nullptr; // optional: the n products g_lo g_hi themselves (byte budget)
-  size_t full_bytes = 0;
+  // optional, forward cosets through matrix passes of a first pass of 2^mm_lr points: its
+  // factors (n rows) and, behind them, its matrices (byte budget)
+  uint64_t* mm_coset = nullptr;
+  int mm_lr = 0;
+  size_t full_bytes = 0;  // of both
   int gs = 0;
 };
 
@@ -1093,7 +1097,8 @@ static int build_roots(const F& f, const TableKey& key, RootTables& t, void** me
   ZKB_TRY(check_launch("NTT inverse stage table"));
   for (int dir = 0; mm && dir < 2; ++dir) {
     t.mm[dir] = reinterpret_cast<unsigned char*>(base) + elems * 32 + dir * kMmDirBytes;
-    k_mm_tables<<<(4096 + kMmTwiddleRows + 127) / 128, 128, 0, s>>>(f, dir ? t.w_inv : t.w_fwd, t.mm[dir]);
+    k_mm_tables<<<(4096 + kMmTwiddleRows + 127) / 128, 128, 0, s>>>(f, dir ? t.w_inv : t.w_fwd, nullptr, nullptr, 0, 0,
+                                                                   t.mm[dir]);
     ZKB_TRY(check_launch("NTT matrix tables"));
   }
   // Other streams may use the entry as soon as it is published.
@@ -1227,10 +1232,9 @@ static int lookup_tables(const F& f, const TableKey& key, int64_t n, int log_n, 
     if (g_scales.size() > kMaxScaleEntries) {
       cudaDeviceSynchronize();
       cudaFree(g_scales.back().mem);
-      if (g_scales.back().t.g_full) {
-        cudaFree(g_scales.back().t.g_full);
-        g_full_bytes -= g_scales.back().t.full_bytes;
-      }
+      cudaFree(g_scales.back().t.g_full);  // freeing null does nothing
+      cudaFree(g_scales.back().t.mm_coset);
+      g_full_bytes -= g_scales.back().t.full_bytes;
       g_scales.pop_back();
     }
   } else {
@@ -1336,12 +1340,52 @@ static int lookup_scale_full(const F& f, int64_t n, int log_n, ScaleTables* st, 
           return rc;
         }
         e.t.g_full = g;
-        e.t.full_bytes = bytes;
+        e.t.full_bytes += bytes;
         g_full_bytes += bytes;
       }
       st->g_full = e.t.g_full;
       break;
     }
+  }
+  return ZKB_OK;
+}
+
+// The factors and matrices of a forward coset's first matrix pass (k_mm_coset), kept in
+// its scale entry (st->mm_coset; null when they do not fit the byte budget, or when the
+// entry holds those of another first pass).
+template <class F>
+static int lookup_scale_mm(const F& f, const RootTables& rt, int64_t n, int lr, int ls, ScaleTables* st,
+                           cudaStream_t s) {
+  st->mm_coset = nullptr;
+  const size_t budget = (size_t)tune_get("ntt.full_table_mb") << 20;
+  const size_t bytes = (size_t)n * 32 + kMmCosetBytes;
+  std::lock_guard<std::mutex> lock(g_ntt_mutex);
+  for (ScaleEntry& e : g_scales) {
+    if (e.t.g_lo != st->g_lo) continue;
+    if (!e.t.mm_coset && g_full_bytes + bytes <= budget) {
+      uint64_t* g = nullptr;
+      ZKB_TRY(check_cuda(cudaMalloc(&g, bytes), "NTT coset factor allocation"));
+      unsigned char* matrices = reinterpret_cast<unsigned char*>(g + 4 * n);
+      uint64_t* inv = reinterpret_cast<uint64_t*>(matrices + kMmMatrixBytes);
+      k_mm_coset_inverses<<<1, 16, 0, s>>>(f, e.t.g_lo, e.t.g_hi, e.t.gs, n, inv);
+      int rc = check_launch("NTT coset factors");
+      k_mm_coset<<<grid_for(n, 128), 128, 0, s>>>(f, rt.w_fwd, e.t.g_lo, e.t.g_hi, e.t.gs, n, lr, ls, inv, g);
+      if (rc == ZKB_OK) rc = check_launch("NTT coset factors");
+      k_mm_tables<<<4096 / 128, 128, 0, s>>>(f, rt.w_fwd, e.t.g_lo, e.t.g_hi, e.t.gs, n, matrices);
+      if (rc == ZKB_OK) rc = check_launch("NTT coset matrices");
+      if (rc == ZKB_OK) rc = check_cuda(cudaStreamSynchronize(s), "NTT coset factor build");
+      if (rc != ZKB_OK) {
+        cudaFree(g);
+        return rc;
+      }
+      e.t.mm_coset = g;
+      e.t.mm_lr = lr;
+      e.t.full_bytes += bytes;
+      g_full_bytes += bytes;
+    }
+    // a budget of 0 means the two-level tables, cached expansions or not
+    if (budget != 0 && e.t.mm_coset && e.t.mm_lr == lr) st->mm_coset = e.t.mm_coset;
+    break;
   }
   return ZKB_OK;
 }
@@ -1519,8 +1563,8 @@ static int launch_pass_tma(const F& f, const PassLaunch& L, int64_t n, int P, in
 // BN254 Fr with the library's tables, every pass of 64, 128 or 256 points on whole
 // 2048-row tiles, at least two tiles for each SM (the blocks are persistent and load
 // 128 KiB of matrices first), and none of the butterfly passes' own knobs set.
-// Measured on B200, butterfly against matrix passes: 2^20 rows 0.250 / 0.237 ms, 2^22
-// 0.916 / 0.722; 2^19 rows are 256 tiles for 148 SMs, two rounds of which the second
+// Measured on B200, butterfly against matrix passes: 2^20 rows 0.250 / 0.221 ms, 2^22
+// 0.919 / 0.660; 2^19 rows are 256 tiles for 148 SMs, two rounds of which the second
 // is three quarters full.
 static bool matrix_passes(const RootTables& rt, const std::vector<PassLaunch>& passes, int64_t n, int sms) {
   if (!rt.mm[0] || tune_get("ntt.matrix") == 0 || (n >> kMmTileLog) < 2 * sms) return false;
@@ -1535,9 +1579,10 @@ static bool matrix_passes(const RootTables& rt, const std::vector<PassLaunch>& p
   return true;
 }
 
-// One pass through k_ntt_pass_mm: its tensor map (a box is C columns of all R rows,
-// one of the two 16-byte halves) and one block per SM.
-static int launch_pass_mm(const FrP& f, const PassLaunch& L, const RootTables& rt, int64_t n, int sms, cudaStream_t s) {
+// One pass through k_ntt_pass_mm: its tensor map (a box is a tile, C columns of all R
+// rows) and one block per SM.
+static int launch_pass_mm(const FrP& f, const PassLaunch& L, const RootTables& rt, const ScaleTables& st, int64_t n,
+                          int sms, cudaStream_t s) {
   NttPass a = L.a;
   a.lc = kMmTileLog - a.lr;
   const uint64_t R = 1ull << a.lr, C = 1ull << a.lc;
@@ -1546,18 +1591,21 @@ static int launch_pass_mm(const FrP& f, const PassLaunch& L, const RootTables& r
     const uint64_t S = 1ull << a.ls, B = R << a.ls;
     const uint64_t dims[4] = {4, S, R, (uint64_t)n / B};
     const uint64_t strides[3] = {32, S * 32, B * 32};
-    const uint32_t box[4] = {2, (uint32_t)C, (uint32_t)R, 1};
-    ZKB_TRY(encode_tensor_map_u64(&map, a.in, 4, dims, strides, box));
+    const uint32_t box[4] = {4, (uint32_t)C, (uint32_t)R, 1};
+    ZKB_TRY(encode_tensor_map_u64(&map, a.in, 4, dims, strides, box, true));
   } else {
     const uint64_t R1 = 1ull << a.lR1, R2 = 1ull << a.lR2;
     const uint64_t dims[4] = {4, R1, R, R2};
     const uint64_t strides[3] = {R2 * R * 32, 32, R * 32};
-    const uint32_t box[4] = {2, (uint32_t)C, (uint32_t)R, 1};
-    ZKB_TRY(encode_tensor_map_u64(&map, a.in, 4, dims, strides, box));
+    const uint32_t box[4] = {4, (uint32_t)C, (uint32_t)R, 1};
+    ZKB_TRY(encode_tensor_map_u64(&map, a.in, 4, dims, strides, box, true));
   }
   constexpr uint32_t mu = FoldTable<FrP>().mu;
-  const MmPass mp{n >> kMmTileLog, rt.mm[a.inverse], mu};
-  const size_t smem = 2 * (size_t)kMmPlane + kMmMatrixBytes + ((size_t)32 << a.lr) + 1024;
+  const uint64_t* coset = a.first && !a.inverse ? st.mm_coset : nullptr;
+  const unsigned char* own = rt.mm[a.inverse];
+  const MmPass mp{n >> kMmTileLog, coset ? reinterpret_cast<const unsigned char*>(coset + 4 * n) : own,
+                  reinterpret_cast<const uint64_t*>(own + kMmMatrixBytes) + 4 * mm_twiddle_row(a.lr), coset, mu};
+  const size_t smem = (size_t)kMmTileBytes + kMmMatrixBytes + ((size_t)32 << a.lr) + 1024;
   ZKB_TRY(check_cuda(cudaFuncSetAttribute(k_ntt_pass_mm<FrP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                      "NTT matrix pass shared memory attribute"));
   ProfSpan span(a.last ? "ntt_last_pass" : "ntt_column_pass", s);
@@ -1576,7 +1624,6 @@ static int run_ntt(const F& f, const zkb_field* field, const uint64_t* in, uint6
   RootTables rt;
   ScaleTables st;
   ZKB_TRY(lookup_tables(f, key, n, log_n, invert, coset, rt, st, s));
-  ZKB_TRY(lookup_scale_full(f, n, log_n, &st, s));
 
   const size_t need = workspace_bytes(n);
   if (need && (!workspace || ws_bytes < need)) {
@@ -1591,6 +1638,15 @@ static int run_ntt(const F& f, const zkb_field* field, const uint64_t* in, uint6
   int sms = 0;
   if (tma) ZKB_TRY(sm_count(device, &sms));
   const bool matrix = tma && matrix_passes(rt, passes, n, sms);
+  if (matrix && st.g_lo && !invert) {
+    ZKB_TRY(lookup_scale_mm(f, rt, n, passes[0].a.lr, passes[0].a.ls, &st, s));
+  } else {
+    st.mm_coset = nullptr;
+  }
+  if (!st.mm_coset) {
+    ZKB_TRY(lookup_scale_full(f, n, log_n, &st, s));
+    for (PassLaunch& L : passes) L.a.g_full = st.g_full;
+  }
   for (int q = 0; q < P; ++q) {
     if (!passes[q].a.last) {
       ZKB_TRY(lookup_twiddles(f, key, rt, passes[q].a.lr, passes[q].a.ls, invert, &passes[q].a.t_full, s));
@@ -1598,7 +1654,7 @@ static int run_ntt(const F& f, const zkb_field* field, const uint64_t* in, uint6
     const PassLaunch& L = passes[q];
     if constexpr (MatrixOk<F>::value) {
       if (matrix) {
-        ZKB_TRY(launch_pass_mm(f, L, rt, n, sms, s));
+        ZKB_TRY(launch_pass_mm(f, L, rt, st, n, sms, s));
         continue;
       }
     }

@@ -206,7 +206,7 @@ static EncodeTiledFn encode_tiled_fn() {
 }
 
 int encode_tensor_map_u64(CUtensorMap* map, const void* base, int rank, const uint64_t* dims,
-                          const uint64_t* strides_bytes, const uint32_t* box) {
+                          const uint64_t* strides_bytes, const uint32_t* box, bool swizzle32) {
   EncodeTiledFn fn = encode_tiled_fn();
   if (!fn) return fail(ZKB_ECUDA, "cuTensorMapEncodeTiled is not available from the driver");
   if (rank < 2 || rank > 5) return fail(ZKB_EINVAL, "tensor map rank %d out of 2..5", rank);
@@ -221,13 +221,15 @@ int encode_tensor_map_u64(CUtensorMap* map, const void* base, int rank, const ui
       return fail(ZKB_EINVAL, "tensor map box dimension %d (%u) out of range", i, box[i]);
     }
   }
+  if (swizzle32 && box[0] * 8u != 32u) return fail(ZKB_EINVAL, "a 32-byte swizzle takes rows of 32 bytes");
   if ((box[0] * 8u) % 16u) return fail(ZKB_EINVAL, "tensor map box inner extent must be a multiple of 16 bytes");
   for (int i = 0; i + 1 < rank; ++i) {
     gstride[i] = strides_bytes[i];
     if (strides_bytes[i] % 16) return fail(ZKB_EINVAL, "tensor map stride %d not a multiple of 16 bytes", i);
   }
   const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT64, (cuuint32_t)rank, const_cast<void*>(base), gdim,
-                        gstride, bdim, estride, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                        gstride, bdim, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        swizzle32 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_NONE,
                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(ZKB_ECUDA, "cuTensorMapEncodeTiled failed (CUresult %d)", (int)r);
   return ZKB_OK;

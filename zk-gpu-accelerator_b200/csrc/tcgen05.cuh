@@ -2,10 +2,12 @@
 // s32 (kind::i8) with both operands in shared memory and the sums in tensor memory.
 //
 // One MMA multiplies A (128 rows of 32 bytes) by B (N rows of 32 bytes, transposed)
-// into 128 lanes by N columns of tensor memory. Both operands are K-major without a
-// swizzle: core matrices of eight rows of 16 bytes, 128 contiguous bytes each;
-// `lbo` bytes lead from a row's first 16 bytes to its second, `sbo` bytes from eight
-// rows to the next eight.
+// into 128 lanes by N columns of tensor memory. Both operands are K-major. Without a
+// swizzle an operand is core matrices of eight rows of 16 bytes, 128 contiguous bytes
+// each: `lbo` bytes lead from a row's first 16 bytes to its second, `sbo` bytes from
+// eight rows to the next eight. With the 32-byte swizzle it is rows of 32 bytes, eight
+// of them contiguous, whose 16-byte halves trade places in rows 4 to 7 (as TMA's
+// 32-byte swizzle lands them).
 #pragma once
 #include <cstdint>
 
@@ -16,6 +18,10 @@ namespace zkb {
 // Shared-memory matrix descriptor (addresses and offsets in 16-byte units).
 __device__ __forceinline__ uint64_t umma_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
   return (uint64_t)((addr >> 4) & 0x3fffu) | (uint64_t)(lbo >> 4) << 16 | (uint64_t)(sbo >> 4) << 32 | 1ull << 46;
+}
+
+__device__ __forceinline__ uint64_t umma_desc_sw32(uint32_t addr, uint32_t sbo) {
+  return umma_desc(addr, 16, sbo) | 6ull << 61;
 }
 
 // Instruction descriptor: u8 operands, s32 sums, both K-major, M = 128 rows.

@@ -86,13 +86,31 @@ __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, u
       : "memory");
 }
 
+// `bytes` (a multiple of 16) contiguous bytes of global memory, both ends 16-byte aligned.
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint64_t* bar, uint32_t bytes) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                   smem_u32(dst)),
+               "l"(src), "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
+}
+
+// The same box into the L2 cache only.
+__device__ __forceinline__ void tma_prefetch_4d(const CUtensorMap* map, int c0, int c1, int c2, int c3) {
+  asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];" ::"l"(
+                   reinterpret_cast<uint64_t>(map)),
+               "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+               : "memory");
+}
+
 // ---- host ------------------------------------------------------------------
 
 // Encodes a tiled tensor map of 64-bit words: rank 2..5, dims[0] innermost
 // (contiguous words), strides_bytes[i] the byte stride of dims[i + 1], box the
-// box extent per dimension. No interleave, no swizzle, no out-of-bounds fill.
+// box extent per dimension. No interleave, no out-of-bounds fill; no swizzle, or
+// (swizzle32, rows of 32 bytes) the 32-byte one: the two 16-byte halves of a row trade
+// places in rows 4 to 7 of every eight.
 // Returns a ZKB status (ZKB_ECUDA with a message when the driver refuses).
 int encode_tensor_map_u64(CUtensorMap* map, const void* base, int rank, const uint64_t* dims,
-                          const uint64_t* strides_bytes, const uint32_t* box);
+                          const uint64_t* strides_bytes, const uint32_t* box, bool swizzle32 = false);
 
 }  // namespace zkb
