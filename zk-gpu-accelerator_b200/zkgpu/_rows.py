@@ -61,6 +61,8 @@ def to_device(x: Any) -> Any:
     """*x* (already shape-checked) as a contiguous torch uint64 tensor on the current CUDA device."""
     torch = _native.require_cuda()
     if isinstance(x, torch.Tensor):
+        if x.is_cuda:
+            return x.contiguous()
         t = x
     elif isinstance(x, np.ndarray):
         t = torch.from_numpy(np.ascontiguousarray(x))

@@ -42,15 +42,15 @@ def _is_pow2(n: int) -> bool:
 def _ntt_jobs(inputs: Sequence[Any], outputs: Sequence[Any], invert: Sequence[bool],
               coset: Sequence[int | None]) -> Any:
     arr = (_native.ZkbNttJob * max(len(inputs), 1))()
-    for j, (x, y, inv, g) in enumerate(zip(inputs, outputs, invert, coset, strict=True)):
-        arr[j].input = _native.ptr(x)
-        arr[j].out = _native.ptr(y)
-        arr[j].n = int(x.shape[0])
-        arr[j].invert = int(bool(inv))
-        arr[j].has_coset = int(g is not None)
+    cosets = {g: tuple(_native.limbs(g % _GROUP_ORDER)) for g in set(coset) if g is not None}
+    for job, x, y, inv, g in zip(arr, inputs, outputs, invert, coset):
+        job.input = x.data_ptr()
+        job.out = y.data_ptr()
+        job.n = x.shape[0]
+        job.invert = int(bool(inv))
         if g is not None:
-            for k, v in enumerate(_native.limbs(g % _GROUP_ORDER)):
-                arr[j].coset[k] = v
+            job.has_coset = 1
+            job.coset = cosets[g]
     return arr
 
 
