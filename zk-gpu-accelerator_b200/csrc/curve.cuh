@@ -439,34 +439,36 @@ __device__ __forceinline__ void sel8(uint32_t r[8], bool c, const uint32_t a[8],
   for (int j = 0; j < 8; ++j) r[j] = c ? a[j] : b[j];
 }
 
-// a := 2a, dbl-2008-s-1 as xyzz_dbl. The identity (ZZ = 0) and Y = 0 both give
-// ZZ = ZZZ = 0 by the formula itself.
+// a := 2a, dbl-2008-s-1 as xyzz_dbl, with M = X (3X) so that the multiples come before
+// the first product. Bounds in units of p beside the steps (fe_mul_open takes a b < 5.29
+// p^2, since 2^256 = 5.29 p, and gives less than a b / 5.29 p + p). The identity (ZZ = 0)
+// and Y = 0 both give ZZ = ZZZ = 0 by the formula itself.
 __device__ __forceinline__ void quad_dbl(uint32_t a[8]) {
   const G1F f;
   const int q = threadIdx.x & 3;
   uint32_t x[8], y[8], s[8], v[8], m[8], t[8], w[8];
-  fe_add(x, a, a, f);
-  sel8(x, q == 1, x, a);   // X, U = 2Y
-  fe_mul(s, x, x, f);      // X^2, V
-  shfl8_quad(v, s, 1);
-  shfl8_quad(w, a, 0);     // X
-  fe_add(m, s, s, f);
-  fe_add(m, m, s, f);      // lane 0: M = 3 X^2
+  add8(x, a, a);            // U = 2Y: 2
+  add8(y, x, a);            // 3X: 3
+  sel8(y, q == 1, x, y);
+  sel8(x, q == 1, x, a);
+  fe_mul_open(m, x, y, f);  // lane 0: M = X 3X, 1.57; lane 1: V = U^2, 1.76
+  shfl8_quad(v, m, 1);
+  shfl8_quad(w, a, 0);      // X
   sel8(x, q >= 2, a, x);
   sel8(x, q == 3, w, x);
   sel8(x, q == 0, m, x);
   sel8(y, q == 0, m, v);
-  fe_mul(t, x, y, f);      // M^2, W = U V, ZZ3 = ZZ V, S = X V
-  shfl8_xor(s, t, 3);      // lane 0: S
-  shfl8_quad(w, t, 1);     // W
+  fe_mul(t, x, y, f);       // M^2 (of 2.5), W = U V (3.6), ZZ3 = ZZ V, S = X V
+  shfl8_xor(s, t, 3);       // lane 0: S
+  shfl8_quad(w, t, 1);      // W
   fe_sub(v, t, s, f);
-  fe_sub(v, v, s, f);      // lane 0: X3 = M^2 - 2S
-  fe_sub(s, s, v, f);      // lane 0: S - X3
+  fe_sub(v, v, s, f);       // lane 0: X3 = M^2 - 2S
+  fe_sub(s, s, v, f);       // lane 0: S - X3
   sel8(x, q == 0, m, a);
   sel8(y, q == 0, s, w);
-  fe_mul(y, x, y, f);      // M (S - X3), W Y, -, ZZZ3 = W ZZZ
+  fe_mul(y, x, y, f);       // M (S - X3), W Y, -, ZZZ3 = W ZZZ
   shfl8_xor(x, y, 1);
-  fe_sub(x, x, y, f);      // lane 1: Y3 = M (S - X3) - W Y
+  fe_sub(x, x, y, f);       // lane 1: Y3 = M (S - X3) - W Y
   sel8(a, q == 2, t, y);
   sel8(a, q == 1, x, a);
   sel8(a, q == 0, v, a);
