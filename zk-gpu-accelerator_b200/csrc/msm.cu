@@ -1100,7 +1100,7 @@ __global__ void __launch_bounds__(kAffThreads, 2) k_msm_affine_round(
 // Three launches whatever the skew, against merge levels of eight slots a thread
 // that took up to ten dependent launches of eight dependent additions. Measured on
 // B200, all merge launches of an MSM: 2^16 points 350 to 125 us, 777,777 skewed
-// scalars 360 to 145 us, 2^22 1.78 to 1.29 ms.
+// scalars 360 to 145 us, 2^22 (runs of 16) 1.78 to 1.29 ms.
 
 struct MergeChunk {
   uint32_t first;  // thread of the first run
@@ -1332,7 +1332,7 @@ __global__ void __launch_bounds__(128) k_msm_reduce(const uint64_t* A_in, const 
 // y = Y / ZZZ with one inversion of ZZ ZZZ, as plain canonical values. About 112
 // dependent doublings at three products each, W - 1 additions at four, and the
 // inversion. One thread took 840 us at 1000 points and 713 us at 2^22 on B200 (187
-// us of it the inversion); this takes 243 and 213 us.
+// us of it the inversion); this takes 233 and 205 us.
 __global__ void __launch_bounds__(32) k_msm_finalize(const MsmJobs J, const uint64_t* all_window_sums, int W,
                                                      int w) {
   const int job = blockIdx.x, q = threadIdx.x & 3;
@@ -1456,14 +1456,15 @@ static int first_level_log(int64_t windows, int64_t nb, int cap) {
   return l;
 }
 
-// The longest automatic run of sorted pairs a bucket thread takes in a one-MSM
-// call ("msm.call_pairs_cap", default 16; batches go up to 64). A bucket block
-// then lasts about 0.5 ms instead of 2 ms at 2^22 points, so kernels the caller
-// runs beside the MSM on other streams (a transform of higher priority) wait at
-// most that long for an SM at each of their launches. Measured on B200, the
-// bench's end-to-end step (two one-call MSMs beside two transforms and their
-// copies): 47.3 to 44.3 ms; the one-call MSM 2^22 alone 18.06 to 18.29 ms.
-static int single_call_pairs_cap() { return tune_get("msm.call_pairs_cap"); }
+// The longest automatic run of sorted pairs in a one-MSM call, twice
+// "msm.call_pairs_cap" (default 16; batches go up to 64). A bucket block then lasts
+// about 0.3 ms at 2^22 points, so kernels the caller runs beside the MSM on other
+// streams (a transform of higher priority) wait at most that long for an SM at each of
+// their launches; the knob's value was the run itself when an addition took twice as
+// long. Longer runs leave fewer of them to
+// merge: at 2^22 points runs of 32 take the merge from 1.28 to 0.66 ms against 16, the
+// bucket kernel the same, on B200.
+static int single_call_pairs_cap() { return 2 * tune_get("msm.call_pairs_cap"); }
 
 // Plan for a batch of jobs with point counts sizes[0..count) at window w.
 static int make_plan(const int64_t* sizes, int count, int w, MsmPlan& p, int table = 0, int k1 = 0,
