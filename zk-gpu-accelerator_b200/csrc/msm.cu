@@ -1253,23 +1253,26 @@ __global__ void __launch_bounds__(256) k_msm_key_ends(const uint32_t* keys, int6
 // item's first bucket. Level 1's items are the buckets themselves (A = T = B,
 // D = 1). One block takes a chunk of 32 L consecutive items of one window, L
 // per quad:
-//   quad t, items j = 0..L-1:  R_t = sum_j T_j,  V_t = sum_j A_j + sum_j j T_j
-//       (running sums from the top: two additions an item, three above level 1)
-//   chunk:  A = sum_t V_t + L sum_t t R_t,  T = 32 L sum_t R_t
-// and sum_t t R_t = sum_(t >= 1) SR_t with SR_t = sum_(u >= t) R_u, a suffix
-// scan across the quads (five additions), then a tree sum of Y_t = V_t + L SR_t
-// (five more). The chunk's pair is the next level's item; a level with one chunk
-// per window writes the window sums. Latency bounds it (some 30 to 50 dependent
-// additions a level on few warps), hence the quads. Measured on B200 against a
-// point per lane, 16 items a lane or quad: 1000 points 359 to 133 us, 2^16 512 to
-// 200 us, 2^22 (eight windows of 2^15 buckets) 585 to 377 us.
+//   quad t, items j = 0..L-1:  R_t = sum_j T_j,  A_t = sum_j A_j + sum_j j T_j
+//       (running sums from the top: two additions an item, three above level 1),
+//       T_t = L R_t
+// and the 32 pairs meet in a tree: of two neighbours l, r that cover the same number of
+// buckets, A = A_l + A_r + T_r (every weight of r grows by that number, which T_r is
+// scaled by) and T = 2 (T_l + T_r). Two additions a step for A, beside T's addition and
+// doubling on the other half of the block. The chunk's pair is the next level's item; a
+// level with one chunk per window writes the window sums. Latency bounds it (some 20
+// to 45 dependent additions a level on few warps), hence the quads. Measured on B200
+// against a point per lane, 16 items a lane or quad: 1000 points 359 to 133 us, 2^16 512
+// to 200 us, 2^22 (eight windows of 2^15 buckets) 585 to 377 us; the tree in place of a
+// suffix scan, a sum and T's doublings at the end (all levels): 1000 points 75 to 67
+// us, 2^16 163 to 135, 2^22 385 to 338, one window of 2^15 buckets 201 to 169 us.
 //
 // A_in / T_in are [W][G_in] (T_in null at level 1: the buckets are both). Out:
 // [W][chunks_per_window] pairs, or (T_out null) the window sums.
 __global__ void __launch_bounds__(128) k_msm_reduce(const uint64_t* A_in, const uint64_t* T_in,
                                                     int64_t G_in, int lL, int64_t chunks_per_window,
                                                     uint64_t* A_out, uint64_t* T_out) {
-  __shared__ __align__(16) uint64_t sm[32 * 16];
+  __shared__ __align__(16) uint64_t sm_a[32 * 16], sm_t[32 * 16];
   const int64_t chunk = blockIdx.x;
   const int t = threadIdx.x >> 2;
   const int64_t win = chunk / chunks_per_window;
@@ -1294,33 +1297,37 @@ __global__ void __launch_bounds__(128) k_msm_reduce(const uint64_t* A_in, const 
     }
     if (k > 0 || !T) quad_add(tot, run);  // level 1: weights 1..L, else 0..L-1 on T
   }
-  // run = R_t, tot = V_t. Suffix scan: run becomes SR_t.
 #pragma unroll 1
-  for (int o = 1; o < 32; o <<= 1) {
-    quad_store(sm + 16 * t, run);
-    __syncthreads();
+  for (int k = 0; k < lL; ++k) quad_dbl(run);
+  quad_store(sm_a + 16 * t, tot);
+  quad_store(sm_t + 16 * t, run);
+  __syncthreads();
+  // 2 h pairs become h: quads 0..h-1 make the A's, quads 16..16+h-1 (other warps) the T's
+  const bool sums = t < 16;
+  const int u = t & 15;
+#pragma unroll 1
+  for (int h = 16; h > 0; h >>= 1) {
+    fe_zero(run);
     fe_zero(x);
-    if (t + o < 32) quad_load(x, sm + 16 * (t + o));
+    fe_zero(tot);
+    if (u < h) {
+      const uint64_t* src = sums ? sm_a : sm_t;
+      quad_load(run, src + 32 * u);
+      quad_load(x, src + 32 * u + 16);
+      if (sums) quad_load(tot, sm_t + 32 * u + 16);
+    }
     __syncthreads();
     quad_add(run, x);
+    if (sums) {
+      quad_add(run, tot);
+    } else {
+      quad_dbl(run);
+    }
+    if (u < h) quad_store((sums ? sm_a : sm_t) + 16 * u, run);
+    __syncthreads();
   }
-  // Y_t = V_t + L SR_t (quad 0 keeps SR_0, the chunk's total)
-  uint32_t sr[8];
-  fe_copy(sr, run);
-#pragma unroll 1
-  for (int k = 0; k < lL; ++k) quad_dbl(sr);
-  fe_zero(x);
-  if (t > 0) fe_copy(x, sr);
-  quad_add(tot, x);
-  quad_block_sum(tot, sm);
-  if (T_out) {
-#pragma unroll 1
-    for (int k = 0; k < 5 + lL; ++k) quad_dbl(run);
-  }
-  if (t == 0) {
-    quad_store(A_out + 16 * chunk, tot);
-    if (T_out) quad_store(T_out + 16 * chunk, run);
-  }
+  if (t == 0) quad_store(A_out + 16 * chunk, run);
+  if (T_out && t == 16) quad_store(T_out + 16 * chunk, run);
 }
 
 // ---------------------------------------------------------------------------
