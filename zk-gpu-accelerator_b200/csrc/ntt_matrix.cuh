@@ -27,15 +27,16 @@
 // beside the workers.
 //
 // What bounds it: the integer multiply pipe. Per row and pass, two twiddle products
-// (136 wide multiply-adds each) and two epilogues of about 20, against 4.25 products
+// (136 wide multiply-adds each) and two epilogues of about 10, against 4.25 products
 // in the radix-4 form: some 20,000 cycles a tile on each scheduler of 27,000 (first
 // and middle passes; the rest is the first half of stage 2's MMAs, 1,000 cycles and
 // their latency, the spread between warps, and in the last pass, whose stage 2 has no
 // product, the load of the next tile). Measured on B200 against the butterfly passes:
-// 2^20 250 to 221 us, 2^22 919 to 660 us, 2^24 3.77 to 2.41 ms, inverse 3.98 to 2.42 ms,
-// coset 4.06 to 2.43 ms. On the way, 2^24: one kind of warp for everything 2.67 ms; with
+// 2^20 231 to 198 us, 2^22 898 to 623 us, 2^24 3.75 to 2.36 ms, inverse 3.96 to 2.35 ms,
+// coset 4.04 to 2.38 ms. On the way, 2^24: one kind of warp for everything 2.67 ms; with
 // the control warp 2.48; the next tile prefetched into L2 2.43; matrices by bulk copy
-// 2.41 (2^20 235 to 221 us). Coset factors as a pass over the tile cost 0.42 ms.
+// 2.41; sums weighed by shifts instead of products by 2^16 2.38. Coset factors as a pass
+// over the tile cost 0.42 ms.
 #pragma once
 #include "tcgen05.cuh"
 
@@ -132,29 +133,39 @@ __global__ void k_mm_coset(F f, const uint64_t* w, const uint64_t* g_lo, const u
   }
 }
 
+// e[0..7] and top += 2^16 sum_j hi[j] 2^(32 j): the odd byte pairs of a row of sums. By
+// shifts and one chain of additions; as products by 2^16 they would take eight slots of
+// the multiply pipe (2^24 forward 2407 to 2380 us; the bucket kernel's reductions, short of
+// registers, lose by it over a table: 1223 to 1243 us).
+__device__ __forceinline__ void add_half_words(uint32_t e[8], uint32_t& top, const uint32_t hi[8]) {
+  uint32_t s[8];
+  s[0] = hi[0] << 16;
+#pragma unroll
+  for (int j = 1; j < 8; ++j) s[j] = __funnelshift_l(hi[j - 1], hi[j], 16);
+  asm("add.cc.u32 %0, %0, %9;\n\t"
+      "addc.cc.u32 %1, %1, %10;\n\t"
+      "addc.cc.u32 %2, %2, %11;\n\t"
+      "addc.cc.u32 %3, %3, %12;\n\t"
+      "addc.cc.u32 %4, %4, %13;\n\t"
+      "addc.cc.u32 %5, %5, %14;\n\t"
+      "addc.cc.u32 %6, %6, %15;\n\t"
+      "addc.cc.u32 %7, %7, %16;\n\t"
+      "addc.u32 %8, %8, %17;"
+      : "+r"(e[0]), "+r"(e[1]), "+r"(e[2]), "+r"(e[3]), "+r"(e[4]), "+r"(e[5]), "+r"(e[6]), "+r"(e[7]), "+r"(top)
+      : "r"(s[0]), "r"(s[1]), "r"(s[2]), "r"(s[3]), "r"(s[4]), "r"(s[5]), "r"(s[6]), "r"(s[7]), "r"(hi[7] >> 16));
+}
+
 // The value of 32 byte-column sums (each at most 256 255^2): sum_m c[m] 2^(8 m) in nine
 // words, below 65280 p when every matrix row is below p.
 __device__ __forceinline__ void mm_weigh(uint32_t v[9], const uint32_t c[32]) {
-  uint32_t e[8], o[8], hi[8], top = 0;
+  uint32_t hi[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
-    e[j] = c[4 * j] + (c[4 * j + 1] << 8);  // below 2^32
+    v[j] = c[4 * j] + (c[4 * j + 1] << 8);  // below 2^32
     hi[j] = c[4 * j + 2] + (c[4 * j + 3] << 8);
   }
-  pairs4(o, hi[1], hi[3], hi[5], hi[7], 65536u);
-  chain4_top(e, top, hi[0], hi[2], hi[4], hi[6], 65536u);
-  v[0] = e[0];
-  asm("add.cc.u32 %0, %8, %16;\n\t"
-      "addc.cc.u32 %1, %9, %17;\n\t"
-      "addc.cc.u32 %2, %10, %18;\n\t"
-      "addc.cc.u32 %3, %11, %19;\n\t"
-      "addc.cc.u32 %4, %12, %20;\n\t"
-      "addc.cc.u32 %5, %13, %21;\n\t"
-      "addc.cc.u32 %6, %14, %22;\n\t"
-      "addc.u32 %7, %15, %23;"
-      : "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8])
-      : "r"(e[1]), "r"(e[2]), "r"(e[3]), "r"(e[4]), "r"(e[5]), "r"(e[6]), "r"(e[7]), "r"(top), "r"(o[0]), "r"(o[1]),
-        "r"(o[2]), "r"(o[3]), "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7]));
+  v[8] = 0;
+  add_half_words(v, v[8], hi);
 }
 
 // r = v mod p in [0, p (1 + 2^-13)), v < 2^271: the quotient's estimate from v's top 32
