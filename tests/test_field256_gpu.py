@@ -146,6 +146,26 @@ def test_raw_rows_with_extreme_words(field):
     assert got == [x * x * rinv % p for x in vals]
 
 
+@pytest.mark.parametrize("multiplier", [0, 1, 2**28 + 1, 2**32 - 1, 2**224, R - 1])
+def test_scalar_products_at_the_quotients_carries(multiplier):
+    """The scalar field's quotient words are shifts (its modulus is 1 - 2^28 mod 2^32) and the low
+    word's carry comes from quotient + word: rows whose words are 0, have an empty or full low nibble,
+    or lie around the modulus's low word, as products and squares."""
+    from zkgpu import _rows
+
+    rng = random.Random(multiplier % 1009)
+    words = (0, 1, 0xF, 0x10, 0x0FFFFFFF, 0x10000000, 0x10000001, 0xEFFFFFFF, 0xF0000000, 0xF0000001, 0xFFFFFFF0)
+    vals = [sum(rng.choice(words) << (32 * w) for w in range(8)) % 2**253 for _ in range(400)]
+    vals += list(words)
+    rinv = pow(2**256, -1, R)
+    a = _rows.upload(_rows.ints_to_limbs(vals))
+    b = _rows.upload(_rows.ints_to_limbs([multiplier] * len(vals)))
+    got = _rows.limbs_to_ints(_rows.download(BN254_FR.mul(a, b)))
+    assert got == [x * multiplier * rinv % R for x in vals]
+    got = _rows.limbs_to_ints(_rows.download(BN254_FR.mul(a, a)))
+    assert got == [x * x * rinv % R for x in vals]
+
+
 def test_operations_compose():
     F, p = BN254_FQ, P
     a, b = operands(p, 4)

@@ -66,6 +66,12 @@ struct FqP {
   __host__ __device__ __forceinline__ static constexpr uint32_t ninv() { return 0xe4866389u; }
 };
 
+// Whether p = 1 - 2^28 mod 2^32 is known when compiling.
+template <class F>
+static constexpr bool kLow28 = false;
+template <>
+constexpr bool kLow28<FrP> = FrP::p(0) == 0xf0000001u;
+
 // Any odd modulus in [3, 2^255), passed by value in kernel parameters
 // (Field256(modulus) for moduli other than BN254's, zkgpu/field256_gpu.py:277-288).
 struct FieldRT {
@@ -278,6 +284,26 @@ __device__ __forceinline__ void chain4(uint32_t o[8], uint32_t a0, uint32_t a1, 
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b));
 }
 
+// e[0..7] += (2^32 - 2^28 + 1, a1, a2, a3) m for m = -e0 (2^28 + 1) mod 2^32, the carry
+// out adds to top. The first pair's low word becomes zero and is not written; its high
+// word grows by floor((m (2^32 - 2^28 + 1) + e0) / 2^32), and as the low word is zero
+// that is m - (m >> 4) plus the carry of m + e0.
+__device__ __forceinline__ void chain4_top_28(uint32_t e[8], uint32_t& top, uint32_t a1, uint32_t a2, uint32_t a3,
+                                              uint32_t m) {
+  uint32_t zero;
+  asm("add.cc.u32 %8, %12, %13;\n\t"
+      "addc.cc.u32 %0, %0, %14;\n\t"
+      "madc.lo.cc.u32 %1, %9, %12, %1;\n\t"
+      "madc.hi.cc.u32 %2, %9, %12, %2;\n\t"
+      "madc.lo.cc.u32 %3, %10, %12, %3;\n\t"
+      "madc.hi.cc.u32 %4, %10, %12, %4;\n\t"
+      "madc.lo.cc.u32 %5, %11, %12, %5;\n\t"
+      "madc.hi.cc.u32 %6, %11, %12, %6;\n\t"
+      "addc.u32 %7, %7, 0;"
+      : "+r"(e[1]), "+r"(e[2]), "+r"(e[3]), "+r"(e[4]), "+r"(e[5]), "+r"(e[6]), "+r"(e[7]), "+r"(top), "=&r"(zero)
+      : "r"(a1), "r"(a2), "r"(a3), "r"(m), "r"(e[0]), "r"(m - (m >> 4)));
+}
+
 // e0 += x, and its carry (from word 0 into word 1) enters the chain
 // o[0..7] += (a0, a1, a2, a3) b, whose first pair is words 1 and 2.
 __device__ __forceinline__ void chain4_in(uint32_t& e0, uint32_t x, uint32_t o[8], uint32_t a0, uint32_t a1,
@@ -327,9 +353,25 @@ struct CiosSum {
   // add m p with m = word 0 (-p^-1) mod 2^32: word 0 becomes zero
   template <class F>
   __device__ __forceinline__ void reduce_row(const F& f) {
-    const uint32_t m = e[0] * f.ninv();
+    const uint32_t m = quotient(e[0], f);
     chain4(o, f.p(1), f.p(3), f.p(5), f.p(7), m);
-    chain4_top(e, top, f.p(0), f.p(2), f.p(4), f.p(6), m);
+    even_row(m, f);
+  }
+
+  // m, and the even words of m p. BN254's scalar field has p = 1 - 2^28 mod 2^32, whose
+  // products are shifts: 56 wide multiply-adds a reduction instead of 64 and 8 narrow
+  // ones (coset NTT 2^24 2372 to 2326 us, 2^12 24.6 to 24.3 us).
+  template <class F>
+  static __device__ __forceinline__ uint32_t quotient(uint32_t e0, const F& f) {
+    if constexpr (kLow28<F>) return 0u - (e0 + (e0 << 28));
+    return e0 * f.ninv();
+  }
+  template <class F>
+  __device__ __forceinline__ void even_row(uint32_t m, const F& f) {
+    if constexpr (kLow28<F>)
+      chain4_top_28(e, top, f.p(2), f.p(4), f.p(6), m);
+    else
+      chain4_top(e, top, f.p(0), f.p(2), f.p(4), f.p(6), m);
   }
 
   // Divide by 2^32 (word 0 is zero): E's pairs move to odd words and O's to even
@@ -589,9 +631,9 @@ __device__ __forceinline__ void fe_sqr(uint32_t r[8], const uint32_t a[8], const
     if (i > 0) {
       const uint32_t x = s.shift();
       const uint32_t m0 = s.e[0] + x;
-      const uint32_t m = m0 * f.ninv();
+      const uint32_t m = CiosSum::quotient(m0, f);
       chain4_in(s.e[0], x, s.o, f.p(1), f.p(3), f.p(5), f.p(7), m);
-      chain4_top(s.e, s.top, f.p(0), f.p(2), f.p(4), f.p(6), m);
+      s.even_row(m, f);
     } else {
       s.reduce_row(f);
     }
