@@ -378,6 +378,28 @@ def test_one_bucket_of_many_runs(runs, sort):
     assert _with_knobs(knobs, lambda: msm_pippenger_rows(same, scalars, window_size=8)) == G * (ks[0] * (n + 3) % R)
 
 
+@pytest.mark.parametrize("window_size", [1, 2, 5, 8, 16])
+@pytest.mark.parametrize("sign", [1, -1])
+def test_window_sums_that_equal_or_cancel_the_doubled_sum(window_size, sign):
+    """The final combination meets its own doubled sum (P = 2^j G with scalar +-1 in one window
+    beside G with scalar 2^j) at the last window and at one before it, where the sum doubles or
+    empties; later windows then go on from there, with and without a point of their own."""
+    for j in range(window_size, 49, window_size):
+        for shift in (0, window_size):
+            pts = [G, G * (1 << j), G * 7]
+            scalars = [1 << (j + shift), sign * (1 << shift) % R, 0]
+            for last in (0, 1):
+                scalars[2] = last
+                want = G * ((scalars[0] + scalars[1] * (1 << j) + 7 * last) % R)
+                got = msm_pippenger_gpu(
+                    np.array([int(p.x) for p in pts], dtype=object),
+                    np.array([int(p.y) for p in pts], dtype=object),
+                    np.array(scalars, dtype=object),
+                    window_size=window_size,
+                )
+                assert got == want, (j, shift, last)
+
+
 # ------------------------------------------------------------------
 # Bucket runs whose products reduce on the tensor cores (the default) against the ones with
 # every product in place (msm.call_products = 0)

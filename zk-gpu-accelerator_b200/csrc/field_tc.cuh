@@ -326,6 +326,20 @@ __device__ __forceinline__ void fold_mul(uint32_t r[8], const uint32_t a[8], con
   fold_reduce(r, t, d, k, f);
 }
 
+// The base field's products of a warp, as a function: canonical results, or (open) those
+// of fold_mul.
+struct FoldMul {
+  FoldWarp k;
+  __device__ __forceinline__ explicit FoldMul(unsigned char* scratch) { k.init(scratch, G1F()); }
+  __device__ __forceinline__ void operator()(uint32_t r[8], const uint32_t a[8], const uint32_t b[8]) const {
+    open(r, a, b);
+    fe_reduce_once(r, G1F());
+  }
+  __device__ __forceinline__ void open(uint32_t r[8], const uint32_t a[8], const uint32_t b[8]) const {
+    fold_mul(r, a, b, nullptr, k, G1F());
+  }
+};
+
 // r = a^2 2^-256 + d; a < 2^255
 template <class F>
 __device__ __forceinline__ void fold_sqr(uint32_t r[8], const uint32_t a[8], const uint32_t* d, const FoldWarp& k,

@@ -1334,44 +1334,281 @@ __global__ void __launch_bounds__(128) k_msm_reduce(const uint64_t* A_in, const 
 // 5. finalize
 // ---------------------------------------------------------------------------
 
-// A warp per job, the chain on quads of lanes (every quad runs the same one).
-// Horner from the top window: acc = 2^w acc + S_win; then affine x = X / ZZ,
-// y = Y / ZZZ with one inversion of ZZ ZZZ, as plain canonical values. About 112
-// dependent doublings at three products each, W - 1 additions at four, and the
-// inversion. One thread took 840 us at 1000 points and 713 us at 2^22 on B200 (187
-// us of it the inversion); this takes 233 and 205 us.
-__global__ void __launch_bounds__(32) k_msm_finalize(const MsmJobs J, const uint64_t* all_window_sums, int W,
-                                                     int w) {
-  const int job = blockIdx.x, q = threadIdx.x & 3;
-  const uint64_t* sums = all_window_sums + 16 * (int64_t)job * W;
+// A warp per job: acc = 2^w acc + S_win from the top window, then x = X / Z^2, y = Y / Z^3
+// with one inversion, as plain canonical values. About 112 dependent doublings, so
+// their depth is what it costs, and the chain's point is kept in a form that doubles in
+// two products instead of three: Jacobian coordinates with v = 3 Z^6 beside them. On the
+// curve X^3 = Y^2 - v, so with t = Y^2 and s = t - v the doubled point (all
+// coordinates scaled by 1/2) is
+//   Z' = Y Z,   X' = X (s / 4 - 2 v),   Y' = 9/8 s (t + 3 v) - t^2,   v' = t^2 (t^2 - s t)
+// Level A makes t, Z' and the v' left open by the doubling before, level B the rest. The
+// products run side by side on eight lanes (q = lane & 7; the four groups do the same):
+//   A: lane 0: Y Y, 1: Y Z, 2: the two factors of v
+//   B: lane 0: (9/8 s) (t + 3 v), 1: s t, 2: t t, 3: X (s / 4 - 2 v), 4: Z Z
+// and a sum with a window's point, kept with its Z, Z^2 and Z^3, takes four more levels.
+// Products are fold_mul's, whose operands may be any 256-bit values, so sums between
+// them are left unreduced; bounds in units of p beside the steps. Measured on B200: one
+// thread 840 us at 1000 points and 713 at 2^22 (187 of it the inversion), XYZZ
+// coordinates on a quad of lanes 237 and 204 us (229 and 198 with these products), this
+// 206 and 176 us.
+struct HornerPoint {
+  uint32_t la[8], lb[8];  // level A's operands: lane 0: Y, Y (at most 3.01); 1: Y, Z; 2: factors of v
+  uint32_t m[8];          // lane 1: Z, 3: X, 4: Z^2
+};
+
+__device__ __forceinline__ void shfl8_oct(uint32_t r[8], const uint32_t a[8], int k) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j) r[j] = __shfl_sync(0xffffffffu, a[j], k, 8);
+}
+
+// r = a / 8 mod p as (a + k p) / 8, k < 8: at most a / 8 + 7/8 p
+__device__ __forceinline__ void fe_eighth(uint32_t r[8], const uint32_t a[8]) {
   const G1F f;
-  uint32_t acc[8], s[8];
-  quad_load(acc, sums + 16 * (W - 1));
-#pragma unroll 1
-  for (int win = W - 2; win >= 0; --win) {
-#pragma unroll 1
-    for (int k = 0; k < w; ++k) quad_dbl(acc);
-    quad_load(s, sums + 16 * win);
-    quad_add(acc, s);
+  const uint32_t k = (a[0] * f.ninv()) & 7;
+  uint32_t e[8], o[8], top = 0;
+  fe_copy(e, a);
+  chain4_top(e, top, f.p(0), f.p(2), f.p(4), f.p(6), k);
+  pairs4(o, f.p(1), f.p(3), f.p(5), f.p(7), k);
+  asm("add.cc.u32 %0, %0, %8;\n\t"
+      "addc.cc.u32 %1, %1, %9;\n\t"
+      "addc.cc.u32 %2, %2, %10;\n\t"
+      "addc.cc.u32 %3, %3, %11;\n\t"
+      "addc.cc.u32 %4, %4, %12;\n\t"
+      "addc.cc.u32 %5, %5, %13;\n\t"
+      "addc.cc.u32 %6, %6, %14;\n\t"
+      "addc.u32 %7, %7, %15;"
+      : "+r"(e[1]), "+r"(e[2]), "+r"(e[3]), "+r"(e[4]), "+r"(e[5]), "+r"(e[6]), "+r"(e[7]), "+r"(top)
+      : "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]), "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7]));
+#pragma unroll
+  for (int j = 0; j < 7; ++j) r[j] = __funnelshift_r(e[j], e[j + 1], 3);
+  r[7] = __funnelshift_r(e[7], top, 3);
+}
+
+// a := 2 a
+__device__ __forceinline__ void horner_dbl(HornerPoint& a, const FoldMul& mul) {
+  const G1F f;
+  const int q = threadIdx.x & 7;
+  uint32_t r[8], t[8], v[8], z[8], s[8], x[8], y[8];
+  mul.open(r, a.la, a.lb);
+  shfl8_oct(t, r, 0);  // 1.01
+  shfl8_oct(v, r, 2);  // 1.01
+  shfl8_oct(z, r, 1);
+  mp_minus<2>(s, v, f);
+  add8(s, s, t);       // s: between 0.99 and 3.01
+  fe_eighth(r, s);     // s / 8: between 0.12 and 1.25
+  sub8(x, r, v);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) y[j] = f.p(j);
+  add8(x, x, y);       // s / 8 - v + p: above 0.1, below 2.3
+  add8(x, x, x);       // s / 4 - 2 v: below 4.6
+  add8(y, v, v);
+  add8(y, y, v);
+  add8(y, y, t);       // t + 3 v: below 4.1
+  add8(r, r, s);       // 9/8 s: below 4.3
+  sel8(r, q == 1, s, r);
+  sel8(r, q == 2, t, r);
+  sel8(r, q == 3, a.m, r);
+  sel8(r, q == 4, z, r);
+  sel8(y, q == 3, x, y);
+  sel8(y, q == 1 || q == 2, t, y);
+  sel8(y, q == 4, z, y);
+  mul.open(r, r, y);
+  sel8(a.m, q == 1, z, r);
+  // lanes 0, 1: Y' = 9/8 s (t + 3 v) - t^2; lane 2: t^2 and t^2 - s t
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    x[j] = __shfl_sync(0xffffffffu, r[j], q == 2 ? 2 : 0, 8);
+    y[j] = __shfl_sync(0xffffffffu, r[j], q == 2 ? 1 : 2, 8);
   }
-  uint32_t zz[8], zzz[8], inv[8], t[8];
-  shfl8_quad(zz, acc, 2);
-  shfl8_quad(zzz, acc, 3);
-  const bool identity = fe_is_zero(zz);
+  mp_minus<2>(y, y, f);
+  add8(y, y, x);       // below 3.01
+  sel8(a.la, q == 2, x, y);
+  sel8(a.lb, q == 1, z, y);
+}
+
+// A window's point (X, Y, ZZ, ZZZ) as Jacobian coordinates with Z = ZZZ: six rows X ZZ^2,
+// Y ZZZ^2, Z, Z^2, Z^3, Z^4 of the table.
+static constexpr int kHornerRow = 6 * 4;
+
+__device__ __forceinline__ void horner_set(HornerPoint& a, const uint64_t* p) {
+  const int q = threadIdx.x & 7;
+  uint32_t zz[8];
+  fe_load(a.m, p + 4 * (q == 1 ? 2 : q == 3 ? 0 : 3));
+  fe_load(a.la, p + 4 * (q == 2 ? 5 : 1));
+  fe_load(a.lb, p + 4 * (q == 1 ? 2 : q == 2 ? 3 : 1));
+  if (q == 2) {  // v = Z^4 (3 Z^2)
+    add8(zz, a.lb, a.lb);
+    add8(a.lb, zz, a.lb);
+  }
+}
+
+// a := a + p, neither the identity, a a doubling's result (Z^2 in lane 4); false: the
+// sum is the identity
+__device__ __forceinline__ bool horner_add(HornerPoint& a, const uint64_t* p, const FoldMul& mul) {
+  const G1F f;
+  const int q = threadIdx.x & 7;
+  uint32_t r[8], x[8], y[8], z[8], u[8], s[8], h[8], hh[8];
+  shfl8_oct(x, a.m, 3);
+  shfl8_oct(y, a.lb, 0);
+  shfl8_oct(z, a.m, 1);
+  shfl8_oct(hh, a.m, 4);
+  fe_load(u, p + 4 * (q == 0 ? 3 : q == 1 ? 0 : q == 2 ? 4 : 2));
+  sel8(r, q == 0, x, z);
+  sel8(r, q == 1 || q == 3, hh, r);
+  sel8(r, q == 2, y, r);
+  sel8(u, q == 3, z, u);
+  mul(r, r, u);          // U1 = X1 ZZ2, U2 = X2 ZZ1, S1 = Y1 ZZZ2, ZZZ1, Z1 Z2
+  shfl8_oct(u, r, 0);
+  shfl8_oct(h, r, 1);
+  shfl8_oct(s, r, 2);
+  shfl8_oct(z, r, 4);
+  shfl8_oct(y, r, 3);
+  fe_sub(h, h, u, f);    // H = U2 - U1
+  fe_load(x, p + 4);
+  sel8(x, q == 1, h, x);
+  sel8(x, q == 2, z, x);
+  sel8(y, q >= 1, h, y);
+  mul(r, x, y);          // S2 = Y2 ZZZ1, HH, Z3 = Z1 Z2 H
+  shfl8_oct(x, r, 0);
+  shfl8_oct(hh, r, 1);
+  shfl8_oct(z, r, 2);
+  fe_sub(y, x, s, f);    // R = S2 - S1
+  if (fe_is_zero(h)) {   // the same in every lane
+    if (!fe_is_zero(y)) return false;
+    horner_dbl(a, mul);
+    return true;
+  }
+  sel8(x, q == 0, h, u);
+  sel8(x, q == 2, y, x);
+  sel8(x, q == 3, z, x);
+  sel8(r, q == 2, y, hh);
+  sel8(r, q == 3, z, r);
+  mul(r, x, r);          // HHH, V = U1 HH, R^2, Z3^2
+  shfl8_oct(h, r, 0);
+  shfl8_oct(u, r, 1);
+  shfl8_oct(x, r, 2);
+  shfl8_oct(hh, r, 3);
+  fe_sub(x, x, h, f);
+  fe_sub(x, x, u, f);
+  fe_sub(x, x, u, f);    // X3 = R^2 - HHH - 2V
+  fe_sub(u, u, x, f);
+  sel8(r, q == 0, y, s);
+  sel8(r, q == 2, hh, r);
+  sel8(u, q == 1, h, u);
+  sel8(u, q == 2, hh, u);
+  mul(r, r, u);          // R (V - X3), S1 HHH, Z3^4
+  shfl8_oct(y, r, 0);
+  shfl8_oct(s, r, 1);
+  fe_sub(y, y, s, f);    // Y3
+  sel8(a.la, q == 2, r, y);
+  add8(u, hh, hh);
+  add8(u, u, hh);        // v3 = Z3^4 (3 Z3^2)
+  sel8(a.lb, q == 1, z, y);
+  sel8(a.lb, q == 2, u, a.lb);
+  sel8(a.m, q == 1, z, hh);
+  sel8(a.m, q == 3, x, a.m);
+  return true;
+}
+
+// The affine point of (x = X or Y, ZZ, ZZZ) from a warp whose even lanes hold X and odd
+// lanes Y, plain and canonical, to `result` (x, y, whether it is the identity).
+__device__ __forceinline__ void store_affine(uint64_t* result, const uint32_t x[8], const uint32_t zz[8],
+                                             const uint32_t zzz[8]) {
+  const G1F f;
+  const int lane = threadIdx.x;
+  uint32_t inv[8], t[8];
+  // one inversion: 1 / ZZ and 1 / ZZZ from that of their product
+  const bool none = fe_is_zero(zz);
   fe_mul(t, zz, zzz, f);
   fe_inv(inv, t, f);
-  sel8(t, q == 0, zzz, zz);
+  sel8(t, (lane & 1) == 0, zzz, zz);
   fe_mul(t, inv, t, f);  // 1 / ZZ, 1 / ZZZ
-  fe_mul(t, acc, t, f);  // x, y
+  fe_mul(t, x, t, f);    // x, y
   fe_from_mont(t, t, f);
-  if (identity) fe_zero(t);
-  uint64_t* result = J.result[job];
+  if (none) fe_zero(t);
   // 8-byte stores: the result buffer only has to be 8-byte aligned
-  if (threadIdx.x < 2) {
+  if (lane < 2) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) result[4 * q + j] = (uint64_t)t[2 * j] | ((uint64_t)t[2 * j + 1] << 32);
+    for (int j = 0; j < 4; ++j) result[4 * lane + j] = (uint64_t)t[2 * j] | ((uint64_t)t[2 * j + 1] << 32);
   }
-  if (threadIdx.x == 0) result[8] = identity ? 1 : 0;
+  if (lane == 0) result[8] = none ? 1 : 0;
+}
+
+__global__ void __launch_bounds__(32) k_msm_finalize(const MsmJobs J, const uint64_t* all_window_sums, int W,
+                                                     int w) {
+  __shared__ __align__(128) unsigned char scratch[kFoldScratch];
+  __shared__ __align__(16) uint64_t table[kHalfBits * kHornerRow];  // a row group per window (w >= 1)
+  const int job = blockIdx.x, lane = threadIdx.x, q = lane & 7;
+  const uint64_t* sums = all_window_sums + 16 * (int64_t)job * W;
+  uint32_t x[8], zz[8], zzz[8], inv[8], t[8];
+  const FoldMul mul(scratch);
+#pragma unroll 1
+  for (int first = 0; first < W; first += 32) {
+    const int win = min(first + lane, W - 1);
+    uint64_t* row = table + kHornerRow * win;
+    fe_load(zz, sums + 16 * win + 8);
+    fe_load(zzz, sums + 16 * win + 12);
+    mul(inv, zz, zz);
+    mul(t, zzz, zzz);
+    fe_load(x, sums + 16 * win);
+    mul(x, x, inv);
+    if (first + lane < W) fe_store(row, x);
+    fe_load(x, sums + 16 * win + 4);
+    mul(x, x, t);
+    mul(inv, t, zzz);
+    mul(zz, t, t);
+    if (first + lane < W) {
+      fe_store(row + 4, x);
+      fe_store(row + 8, zzz);
+      fe_store(row + 12, t);
+      fe_store(row + 16, inv);
+      fe_store(row + 20, zz);
+    }
+  }
+  __syncwarp();
+  HornerPoint acc;
+  bool identity = true;  // no point yet; the same in every lane, as all branches here
+#pragma unroll 1
+  for (int win = W - 1; win >= 0; --win) {
+    const uint64_t* row = table + kHornerRow * win;
+    if (!identity) {
+#pragma unroll 1
+      for (int k = 0; k < w; ++k) horner_dbl(acc, mul);
+    }
+    fe_load(t, row + 8);
+    if (fe_is_zero(t)) continue;
+    if (identity) {
+      horner_set(acc, row);
+      identity = false;
+    } else {
+      identity = !horner_add(acc, row, mul);
+    }
+  }
+  if (identity) {
+    fe_zero(x);
+    fe_zero(zz);
+    fe_zero(zzz);
+  } else {
+    uint32_t y[8];
+    shfl8_oct(x, acc.m, 3);
+    shfl8_oct(y, acc.lb, 0);
+    sel8(x, q & 1, y, x);
+    shfl8_oct(t, acc.m, 1);
+    mul(zz, t, t);
+    mul(zzz, zz, t);
+  }
+  store_affine(J.result[job], x, zz, zzz);
+}
+
+// One window (a fixed-base table): its sum is the result. In a kernel of its own, 26 us
+// against 32 as a branch of k_msm_finalize.
+__global__ void __launch_bounds__(32) k_msm_finalize_one(const MsmJobs J, const uint64_t* all_window_sums) {
+  const uint64_t* sum = all_window_sums + 16 * (int64_t)blockIdx.x;
+  uint32_t x[8], zz[8], zzz[8];
+  fe_load(x, sum + 4 * (threadIdx.x & 1));
+  fe_load(zz, sum + 8);
+  fe_load(zzz, sum + 12);
+  store_affine(J.result[blockIdx.x], x, zz, zzz);
 }
 
 __global__ void k_msm_identity_result(uint64_t* result) {
@@ -1826,7 +2063,11 @@ static int run_msm(const MsmJobs& J, const MsmPlan& p, char* ws, cudaStream_t s)
   // 5. finalize
   ProfSpan fin_span("msm_finalize", s);
   // with tables there is one window sum per job: nothing to combine
-  k_msm_finalize<<<(unsigned)p.count, 32, 0, s>>>(J, wsum, p.table ? 1 : p.W, p.w);
+  if (p.table || p.W == 1) {
+    k_msm_finalize_one<<<(unsigned)p.count, 32, 0, s>>>(J, wsum);
+  } else {
+    k_msm_finalize<<<(unsigned)p.count, 32, 0, s>>>(J, wsum, p.W, p.w);
+  }
   return check_launch("msm finalize");
 }
 
