@@ -114,10 +114,16 @@ def _peaks() -> dict:
 # Work accounting
 # ------------------------------------------------------------------
 
-IMAD_PER_MULMOD = 264  # 2 x 64 32-bit multiply-adds (lo and hi) for a*b and m*p, plus 8 for the m's
-IMAD_PER_SQR = 208     # 2 x (36 + 64) for a*a (each cross product once) and m*p, plus 8 for the m's
-# XYZZ mixed addition: 8 multiplications + 2 squarings
-IMAD_PER_MADD = 8 * IMAD_PER_MULMOD + 2 * IMAD_PER_SQR
+# 32-bit multiply-adds (lo and hi) that the kernels issue. A reduction on the tensor cores
+# (csrc/field_tc.cuh) leaves 18 wide multiply-adds of the 64 + 8 that m's and m*p take.
+IMAD_PER_FOLD = 2 * 18
+IMAD_PER_MULMOD = 2 * 64 + IMAD_PER_FOLD  # a*b
+IMAD_PER_SQR = 2 * 36 + IMAD_PER_FOLD     # a*a (each cross product once)
+# XYZZ mixed addition: 8 multiplications, two of them sharing a reduction, and 2 squarings
+IMAD_PER_MADD = 8 * IMAD_PER_MULMOD - IMAD_PER_FOLD + 2 * IMAD_PER_SQR
+# a scalar-field product of the transforms: a*b and 56 for the reduction (csrc/field.cuh)
+IMAD_PER_NTT_PRODUCT = 2 * (64 + 56)
+NTT_MATRIX_MIN_LOG = 20  # transforms from 2^20 rows run as byte matrix products (csrc/ntt_matrix.cuh)
 PRODUCTS_PER_MADD = 10
 
 
@@ -145,6 +151,18 @@ def ntt_products(n: int, log_n: int, passes: int | None = None) -> int:
         per_row += (0.25 + (rounds - 1) if rounds else 0.0) + (0.5 if lr % 2 and lr > 1 else 0.0)
     per_row += P - 1
     return int(per_row * n)
+
+
+def ntt_imads(n: int, log_n: int, passes: int) -> tuple[int, int]:
+    """(products, 32-bit multiply-adds) of one forward NTT as csrc/ntt.cu runs it. Matrix passes
+    (csrc/ntt_matrix.cuh) multiply each row by an internal twiddle in every pass and by a boundary
+    twiddle in all but the last, and reduce two matrix sums a row and pass (9 wide multiply-adds
+    each); the sums themselves are on the tensor cores."""
+    if log_n < NTT_MATRIX_MIN_LOG:
+        products = ntt_products(n, log_n, passes)
+        return products, products * IMAD_PER_NTT_PRODUCT
+    products = n * (2 * passes - 1)
+    return products, products * IMAD_PER_NTT_PRODUCT + n * 2 * passes * 2 * 9
 
 
 def _glv_halves(k: int) -> tuple[int, int]:
@@ -536,7 +554,8 @@ def run_ours(args, rank: int, world: int, local_rank: int) -> dict | None:
             "products_frac_of_measured": round(products / (ms * 1e-3) / prod_meas, 4),
             "peak_source": f"nominal issue rate: {sm_count} SMs x 64 IMAD/clk x {mhz:.0f} MHz (median SM clock "
                            "sampled in the timed region)",
-            "work_per_launch": f"{madds} mixed additions x (8 x {IMAD_PER_MULMOD} + 2 x {IMAD_PER_SQR}) IMAD",
+            "work_per_launch": f"{madds} mixed additions x {IMAD_PER_MADD} IMAD issued (8 products and 2 squarings, "
+                               "their reductions on the tensor cores)",
             "launch_ms": round(ms, 4), "launches": count,
             "hbm": {"achieved": round(acc_bytes / (ms * 1e-3) / 1e9, 1), "peak": hbm_peak, "unit": "GB/s",
                     "frac": round(acc_bytes / (ms * 1e-3) / 1e9 / hbm_peak, 4) if hbm_peak else None,
@@ -557,22 +576,23 @@ def run_ours(args, rank: int, world: int, local_rank: int) -> dict | None:
 
     traffic_u = _profile_traffic("k_msm_acc_points", step.n)
     traffic_s = _profile_traffic("k_msm_acc_points_skewed", step.n)
-    # the step's own launch (both MSMs' pairs, k_msm_acc_points_batch), timed live in the
+    # the step's own launch (both MSMs' pairs, k_msm_acc_points_tc<true>), timed live in the
     # timed region while the transforms run beside it on the low-priority stream
     roofline = acc_roof(madds_u + madds_s, prof_live,
-                        "k_msm_acc_points_batch (bucket accumulation of both MSMs of the step, live)",
+                        "k_msm_acc_points_tc<true> (bucket accumulation of both MSMs of the step, live)",
                         traffic_u + traffic_s if traffic_u and traffic_s else None)
     # the uniform MSM's launch alone (one call, nothing beside it)
-    roofline_alone = acc_roof(madds_u, prof_msm, "k_msm_acc_points (uniform scalars, one call alone)", traffic_u)
+    roofline_alone = acc_roof(madds_u, prof_msm, "k_msm_acc_points_tc<false> (uniform scalars, one call alone)",
+                              traffic_u)
     # NTT passes: bytes moved (read + write of 32-byte rows per pass) against HBM
     ntt_pass_ms = sum(v[1] for k, v in prof_ntt.items() if k.startswith("ntt_")) / max(2, min(args.steps, 5))
     n_passes = sum(v[0] for k, v in prof_ntt.items() if k.startswith("ntt_")) / max(2, min(args.steps, 5))
     ntt_bytes = 64 * step.m * n_passes
     ntt_gbs = ntt_bytes / (ntt_pass_ms * 1e-3) / 1e9
-    ntt_mulmods = ntt_products(step.m, log_ntt, round(n_passes) or None)
+    ntt_mulmods, ntt_imad = ntt_imads(step.m, log_ntt, round(n_passes) or 3)
     ntt_roof = {"bytes_per_launch": int(ntt_bytes), "ms": round(ntt_pass_ms, 4), "achieved_gbs": round(ntt_gbs, 1),
                 "hbm_frac": round(ntt_gbs / hbm_peak, 4) if hbm_peak else None,
-                "imad_frac": round(ntt_mulmods * IMAD_PER_MULMOD / (ntt_pass_ms * 1e-3) / 1e12 / imad_peak_t, 4),
+                "imad_frac": round(ntt_imad / (ntt_pass_ms * 1e-3) / 1e12 / imad_peak_t, 4),
                 "products": ntt_mulmods, "passes": n_passes}
 
     # ---- end to end through the public API, pinned host buffers, copies inside the timed region

@@ -3,9 +3,10 @@
 //
 // Pipeline for sum_i s_i P_i (zkgpu/msm_gpu.py:1-35 describes the reference's
 // version; here every step, including the final combination, is on the GPU):
-//   1. digits    one thread per scalar: reduce mod r, recode into W signed
-//                w-bit digits d (|d| <= 2^(w-1)), and emit one (bucket, point)
-//                pair per nonzero digit: key = window * 2^(w-1) + |d| - 1,
+//   1. digits    one thread per scalar: reduce mod r, split into two GLV halves, phi(P);
+//                then one thread per half and window: the signed w-bit digit d
+//                (|d| <= 2^(w-1)), and one (bucket, point) pair per nonzero
+//                digit: key = window * 2^(w-1) + |d| - 1,
 //                value = point index | sign << 31.
 //   2. sort      group the pairs by key, so every bucket's points are
 //                contiguous: either a counting sort ("msm.sort" = 1): the
@@ -15,7 +16,7 @@
 //                into its bucket's range; or a radix sort of all 2 W n pairs by key (CUB
 //                onesweep, "msm.sort" = 0), zero digits carrying the largest
 //                key and sorting to the end.
-//   3. buckets   level 1: each thread adds a fixed run of K1 sorted pairs into
+//   3. buckets   each thread adds a fixed run of K1 sorted pairs into
 //                XYZZ accumulators with mixed additions, so every thread does
 //                the same work however skewed the buckets are. A bucket wholly
 //                inside one thread's run is written out directly; a bucket
@@ -23,15 +24,9 @@
 //                slots, which a merge adds per bucket (full XYZZ additions on
 //                quads of lanes; large buckets in chunks). No host sync.
 //   4. reduction sum_b (b + 1) B_b per window by running sums over segments of
-//                L buckets, recursively over the segment sums (below).
+//                L buckets and a tree over the segments' pairs (below).
 //   5. finalize  Horner over the window sums (w doublings per window) and one
 //                inversion to affine (zkgpu/msm.py:156-169, curve.py:221-233).
-//
-// Window-sum recursion: for a segment t of L consecutive entries X_{tL+i},
-// running sums from the top give S_t = sum_i X_{tL+i} and
-// U_t = sum_i (i + delta) X_{tL+i}; then
-//   sum_b (b + delta) X_b = sum_t U_t + L * sum_t t S_t,
-// and the last term is the same problem on the L S_t with delta = 0.
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 
@@ -749,7 +744,7 @@ __global__ void __launch_bounds__(128, 4) k_msm_acc_points_tc(const MsmJobs J, c
 // points (signs applied); later rounds read the previous round's points. The
 // bucket layout of a round is its list of bucket ends (an inclusive scan of
 // the halved counts). After the last round, the short lists go through the
-// XYZZ run and merge levels as (bucket, entry) pairs.
+// XYZZ runs and merge as (bucket, entry) pairs.
 //
 // The sharing is per block and pipelined. Warps 0..6 are workers: in a batch
 // each worker thread chains the denominators of its k output entries into one
@@ -1666,7 +1661,7 @@ struct MsmPlan {
   int aff_k = 64;                   // output entries per thread of an affine round ("msm.affine_batch")
   std::vector<int64_t> aff_bound;   // bound on each round's list: aff_bound[0] = E, then per round
   int64_t E_list = 0;               // entries the XYZZ levels start from (E, or the last round's bound)
-  int64_t T1 = 0;  // level-1 threads
+  int64_t T1 = 0;  // bucket threads
   uint32_t merge_thr = 0;   // the most runs a bucket's quad adds by itself
   int64_t max_chunks = 0;   // bound on the merge chunks of larger buckets
   size_t cub_bytes = 0;
@@ -1750,9 +1745,9 @@ static int make_plan(const int64_t* sizes, int count, int w, MsmPlan& p, int tab
   }
   p.aff_rounds = (int)p.aff_bound.size() - 1;
   p.E_list = p.aff_bound.back();
-  // pairs per level-1 thread: the knob, else by size. A thread adds its pairs one
+  // pairs per bucket thread: the knob, else by size. A thread adds its pairs one
   // after another, so small MSMs want short chains and many threads; each thread
-  // may leave two partial sums for the merge levels, so large ones want long
+  // may leave two partial sums for the merge, so large ones want long
   // chains. E / 2^19 rounded down to a power of two, within 8..64: measured on
   // B200 (uniform scalars, default windows), 8 pairs against 64 take 2^10 points
   // from 1.89 to 1.56 ms, 2^14 from 2.07 to 1.79, 2^16 from 2.36 to 2.14; from

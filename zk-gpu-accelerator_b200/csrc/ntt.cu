@@ -1563,8 +1563,8 @@ static int launch_pass_tma(const F& f, const PassLaunch& L, int64_t n, int P, in
 // BN254 Fr with the library's tables, every pass of 64, 128 or 256 points on whole
 // 2048-row tiles, at least two tiles for each SM (the blocks are persistent and load
 // 128 KiB of matrices first), and none of the butterfly passes' own knobs set.
-// Measured on B200, butterfly against matrix passes: 2^20 rows 0.250 / 0.221 ms, 2^22
-// 0.919 / 0.660; 2^19 rows are 256 tiles for 148 SMs, two rounds of which the second
+// Measured on B200, butterfly against matrix passes: 2^20 rows 0.231 / 0.198 ms, 2^22
+// 0.898 / 0.623; 2^19 rows are 256 tiles for 148 SMs, two rounds of which the second
 // is three quarters full.
 static bool matrix_passes(const RootTables& rt, const std::vector<PassLaunch>& passes, int64_t n, int sms) {
   if (!rt.mm[0] || tune_get("ntt.matrix") == 0 || (n >> kMmTileLog) < 2 * sms) return false;

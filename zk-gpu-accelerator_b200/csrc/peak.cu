@@ -6,7 +6,10 @@
 // Three loops, each over independent chains so that the pipe, not latency,
 // bounds them, in blocks of 256 threads:
 //   mad.lo.u32     a = a * m + c, 8 chains per thread
-//   mad.wide.u32   A = x * y + A (32 x 32 -> 64 bits), 8 chains per thread
+//   mad.wide.u32   A = x * y + A (32 x 32 -> 64 bits), 8 chains per thread; x and y stay,
+//                  so the product leaves the loop and this is the rate of its 64-bit
+//                  additions (a multiply-add whose factors change issues 32 lanes per SM
+//                  per clock on B200)
 //   Montgomery     x = x * y mod q over BN254's base field (fe_mul, inline),
 //                  4 chains per thread
 // Each launch is one wave: as many 256-thread blocks per SM as fit at once
