@@ -574,8 +574,8 @@ def run_ours(args, rank: int, world: int, local_rank: int) -> dict | None:
                   "mad.wide.u32 and 256-bit Montgomery products, SM cycle counters; scaled to the clock "
                   "sampled in the timed region"}
 
-    traffic_u = _profile_traffic("k_msm_acc_points", step.n)
-    traffic_s = _profile_traffic("k_msm_acc_points_skewed", step.n)
+    traffic_u = _profile_traffic("k_msm_acc_points_tc", step.n)
+    traffic_s = _profile_traffic("k_msm_acc_points_tc_skewed", step.n)
     # the step's own launch (both MSMs' pairs, k_msm_acc_points_tc<true>), timed live in the
     # timed region while the transforms run beside it on the low-priority stream
     roofline = acc_roof(madds_u + madds_s, prof_live,
