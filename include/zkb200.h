@@ -97,9 +97,10 @@ int zkb_field_from_mont(const zkb_field* f, const uint64_t* in, uint64_t* out, i
 /* Device workspace (bytes) zkb_ntt needs for a transform of n rows. */
 size_t zkb_ntt_workspace_bytes(int64_t n);
 
-/* Number of NTT pass tiles on the current device, since the library loaded,
- * whose bounded wait for their TMA loads gave up (each such block stops early
- * and that transform's output is incomplete); 0 in a healthy run. It has no
+/* Number of NTT pass blocks on the current device, since the library loaded,
+ * in which a bounded wait (for a tile's TMA loads; in a matrix pass, any of its
+ * waits) gave up: each such block stops early and that transform's output is
+ * incomplete; 0 in a healthy run. It has no
  * counterpart in the reference. Synchronous; ~0 if the device cannot be read. */
 uint64_t zkb_ntt_wait_timeouts(void);
 
@@ -365,7 +366,10 @@ int zkb_msm_fixed_batch(const zkb_msm_job* jobs, int count, void* workspace, siz
  * every operation; the same rows either way), "ntt.matrix" (1: transforms of
  * 2^20 to 2^24 rows over BN254's Fr run passes of 64 to 256 points as byte matrix
  * products on the tensor cores, while the knobs of the butterfly passes are at their
- * defaults; 0: butterfly passes; the same rows either way);
+ * defaults; 0: butterfly passes; the same rows either way), "ntt.matrix_polls"
+ * (polls of such a pass's first wait, for its matrices, before it gives up, its
+ * block stops early and zkb_ntt_wait_timeouts counts it; 0 = the default 2^24, as
+ * for every other wait, -1 = none at all);
  * "msm.affine_rounds" (rounds in which every bucket's list is halved by affine
  * additions sharing one inversion per block, before the XYZZ levels; 0 = none,
  * the default; -1 = by size; 1..8 forced), "msm.affine_batch" (output entries

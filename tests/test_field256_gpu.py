@@ -486,3 +486,43 @@ def test_matrix_passes_equal_butterfly_passes(log_n, table_mb):
         _native.tune_set("ntt.matrix", 1)
         _native.tune_set("ntt.full_table_mb", 4096)
     assert lib.zkb_ntt_wait_timeouts() == 0
+
+
+_WAITS_THAT_RUN_OUT = """
+import torch
+from zkgpu import _native, workloads as wl
+from zkgpu.field256_gpu import BN254_FR
+
+lib = _native.lib()
+sms = torch.cuda.get_device_properties(0).multi_processor_count
+rows = BN254_FR.to_montgomery(wl.uniform_fr(520, 1 << 20))
+_native.tune_set("ntt.matrix", 0)
+want = {c: BN254_FR.ntt(rows, coset=c) for c in (None, 5)}
+_native.tune_set("ntt.matrix", 1)
+for coset in (None, 5):
+    before = lib.zkb_ntt_wait_timeouts()
+    _native.tune_set("ntt.matrix_polls", -1)
+    BN254_FR.ntt(rows, coset=coset)
+    torch.cuda.synchronize()
+    assert lib.zkb_ntt_wait_timeouts() - before == 3 * sms  # each block of three passes, once
+    _native.tune_set("ntt.matrix_polls", 0)
+    assert bool((BN254_FR.ntt(rows, coset=coset) == want[coset]).all())
+    assert lib.zkb_ntt_wait_timeouts() - before == 3 * sms
+print("ok")
+"""
+
+
+def test_matrix_pass_waits_that_run_out_are_counted_and_leave_the_gpu_usable():
+    """With no polls ("ntt.matrix_polls" = -1) the control lane's first wait gives up at once and the
+    worker warps' waits follow: each block counts itself once, lets its loads land and returns; the
+    next transform is exact again.
+    In a process of its own: the count is the library's and other tests want it to be 0."""
+    import subprocess
+    import sys
+
+    from conftest import ROOT
+
+    env = {**os.environ, "PYTHONPATH": str(ROOT / "zk-gpu-accelerator_b200")}
+    out = subprocess.run([sys.executable, "-c", _WAITS_THAT_RUN_OUT], env=env, capture_output=True, text=True,
+                         timeout=300)
+    assert out.returncode == 0 and out.stdout.strip() == "ok", out.stderr

@@ -1603,8 +1603,10 @@ static int launch_pass_mm(const FrP& f, const PassLaunch& L, const RootTables& r
   constexpr uint32_t mu = FoldTable<FrP>().mu;
   const uint64_t* coset = a.first && !a.inverse ? st.mm_coset : nullptr;
   const unsigned char* own = rt.mm[a.inverse];
+  const int knob = tune_get("ntt.matrix_polls");
+  const uint32_t polls = knob == 0 ? kTmaWaitLimit : knob < 0 ? 0u : (uint32_t)knob;
   const MmPass mp{n >> kMmTileLog, coset ? reinterpret_cast<const unsigned char*>(coset + 4 * n) : own,
-                  reinterpret_cast<const uint64_t*>(own + kMmMatrixBytes) + 4 * mm_twiddle_row(a.lr), coset, mu};
+                  reinterpret_cast<const uint64_t*>(own + kMmMatrixBytes) + 4 * mm_twiddle_row(a.lr), coset, mu, polls};
   const size_t smem = (size_t)kMmTileBytes + kMmMatrixBytes + ((size_t)32 << a.lr) + 1024;
   ZKB_TRY(check_cuda(cudaFuncSetAttribute(k_ntt_pass_mm<FrP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                      "NTT matrix pass shared memory attribute"));

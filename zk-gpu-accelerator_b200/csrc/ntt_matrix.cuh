@@ -248,17 +248,40 @@ struct MmPass {
   const uint64_t* twiddles;     // internal twiddles [k1][j0]
   const uint64_t* coset;        // k_mm_coset's factors in their place (null: none)
   uint32_t mu;                  // floor(2^285 / p)
+  uint32_t polls;               // of the wait for the matrices, before it gives up
 };
 
-// Waits for a phase of `bar`; false once the wait or any other of the block has run
-// out of polls.
-__device__ __forceinline__ bool mm_wait(uint64_t* bar, uint32_t parity, volatile int* failed) {
-  for (uint32_t i = 0; i < kTmaWaitLimit; ++i) {
+// A wait of the block has run out of polls: the first to say so counts the block.
+__device__ __forceinline__ void mm_give_up(int* failed) {
+  if (atomicExch(failed, 1) == 0) atomicAdd(&g_ntt_tma_timeouts, 1u);
+}
+
+// The control lane's wait for a phase of `bar`; false once it or any other wait of the
+// block has run out of polls.
+__device__ __forceinline__ bool mm_wait(uint64_t* bar, uint32_t parity, uint32_t polls, int* failed) {
+  for (uint32_t i = 0; i < polls; ++i) {
     if (mbar_try_wait(bar, parity)) return true;
-    if ((i & 255u) == 255u && *failed) return false;
+    if ((i & 255u) == 255u && *(volatile int*)failed) return false;
   }
-  *failed = 1;
+  mm_give_up(failed);
   return false;
+}
+
+// The same for a whole worker warp. The lanes' answers are one vote a poll, so that they
+// leave together: what follows a wait is collective (tcgen05.ld.sync.aligned), and a lane
+// that gave up alone would leave the others in it. (The vote costs nothing that shows, 2^24
+// coset 2325 and 2321 us; a vote after each lane's own polls 2 %, and a limit that is no
+// constant 40 bytes of spills.)
+__device__ __forceinline__ bool mm_wait_warp(uint64_t* bar, uint32_t parity, int* failed) {
+  for (uint32_t i = 0; !__all_sync(0xffffffffu, mbar_try_wait(bar, parity)); ++i) {
+    if ((i & 255u) != 255u) continue;
+    const bool late = i >= kTmaWaitLimit;
+    if (__any_sync(0xffffffffu, late || *(volatile int*)failed)) {
+      if (late) mm_give_up(failed);
+      return false;
+    }
+  }
+  return true;
 }
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
@@ -272,7 +295,8 @@ __global__ void __launch_bounds__(kMmThreads, 1) k_ntt_pass_mm(F f, const NttPas
   unsigned char* sm = smem_raw_mm + ((1024u - (smem_u32(smem_raw_mm) & 1023u)) & 1023u);
   // the matrices have landed; the tile has; its coset factors are in; the MMAs of half h of a stage are
   // done; the tile holds stage 2's rows; half h of stage 2's sums has been read
-  __shared__ __align__(8) uint64_t s_matrix, s_load, s_scaled, s_mma[2], s_rows, s_read[2];
+  // (s_drain: the MMAs in flight are done, after a wait that gave up)
+  __shared__ __align__(8) uint64_t s_matrix, s_load, s_scaled, s_mma[2], s_rows, s_read[2], s_drain;
   __shared__ uint32_t s_tmem;
   __shared__ int s_failed;
   const int lr = a.lr, lc = a.lc, l2 = lr - 4, C = 1 << lc, r2 = 1 << l2;
@@ -302,6 +326,7 @@ __global__ void __launch_bounds__(kMmThreads, 1) k_ntt_pass_mm(F f, const NttPas
     mbar_init(&s_load, 1);
     mbar_init(&s_scaled, kMmWorkers);
     mbar_init(&s_rows, kMmWorkers);
+    mbar_init(&s_drain, 1);
     for (int h = 0; h < 2; ++h) {
       mbar_init(&s_mma[h], 1);
       mbar_init(&s_read[h], kMmWorkers);
@@ -339,14 +364,16 @@ __global__ void __launch_bounds__(kMmThreads, 1) k_ntt_pass_mm(F f, const NttPas
         }
       };
       bool ok = true;
-      uint32_t round = 0;  // tiles done
+      bool loading = true;  // tile `round` is on its way
+      uint32_t round = 0;   // tiles done
       mbar_arrive_expect_tx(&s_matrix, kMmMatrixBytes);
       for (int i = 0; i < 4; ++i)
         bulk_load(mat + i * (kMmMatrixBytes / 4), mp.matrices + i * (kMmMatrixBytes / 4), &s_matrix, kMmMatrixBytes / 4);
       if (blockIdx.x < mp.ntiles) issue_load(blockIdx.x);
-      ok = mm_wait(&s_matrix, 0, &s_failed);
+      const bool matrices = ok = mm_wait(&s_matrix, 0, mp.polls, &s_failed);
       for (int64_t tile = blockIdx.x; tile < mp.ntiles && ok; tile += gridDim.x, ++round) {
-        ok = mm_wait(&s_load, round & 1, &s_failed);
+        if (!(ok = mm_wait(&s_load, round & 1, kTmaWaitLimit, &s_failed))) break;
+        loading = false;
         if (tile + gridDim.x < mp.ntiles) {
           // the next tile into L2 meanwhile: from memory its load took 6,600 cycles, more
           // than what is left of this tile when it may start
@@ -354,11 +381,11 @@ __global__ void __launch_bounds__(kMmThreads, 1) k_ntt_pass_mm(F f, const NttPas
           box(tile + gridDim.x, x1, x3);
           tma_prefetch_4d(&tmap, 0, x1, 0, x3);
         }
-        if (ok && prescale) ok = mm_wait(&s_scaled, round & 1, &s_failed);
+        if (prescale) ok = mm_wait(&s_scaled, round & 1, kTmaWaitLimit, &s_failed);
         // stage 1: rows (j0, c), 16 points over j1, 128 indices apart. Half h may start
         // once half h of the last tile's sums has been read.
         for (int h = 0; h < 2 && ok; ++h) {
-          if (round > 0) ok = mm_wait(&s_read[h], (round - 1) & 1, &s_failed);
+          if (round > 0) ok = mm_wait(&s_read[h], (round - 1) & 1, kTmaWaitLimit, &s_failed);
           if (!ok) break;
           tmem_fence_after();
           mma_run(h * 128, 0, 256, 0, 1, 8, 4 * h, 128);          // E_k: rows j1 = 0, 2, ..
@@ -366,7 +393,7 @@ __global__ void __launch_bounds__(kMmThreads, 1) k_ntt_pass_mm(F f, const NttPas
           umma_commit(&s_mma[h]);
         }
         // stage 2: rows (k1, c), r2 points over j0, 16 C indices apart
-        if (!ok || !(ok = mm_wait(&s_rows, round & 1, &s_failed))) break;
+        if (!ok || !(ok = mm_wait(&s_rows, round & 1, kTmaWaitLimit, &s_failed))) break;
         tmem_fence_after();
         const uint32_t dist = 16u << lc;
         if (r2 == 16) {
@@ -385,15 +412,19 @@ __global__ void __launch_bounds__(kMmThreads, 1) k_ntt_pass_mm(F f, const NttPas
           }
         }
         // the tile's memory is free once both halves are done
-        ok = mm_wait(&s_mma[1], 1, &s_failed);
-        if (ok && tile + gridDim.x < mp.ntiles) issue_load(tile + gridDim.x);
+        ok = mm_wait(&s_mma[1], 1, kTmaWaitLimit, &s_failed);
+        if (ok && tile + gridDim.x < mp.ntiles) {
+          issue_load(tile + gridDim.x);
+          loading = true;
+        }
       }
       if (!ok) {
-        // a wait gave up: record it, and let loads and MMAs in flight land (bounded)
-        atomicAdd(&g_ntt_tma_timeouts, 1u);
-        mbar_wait_bounded(&s_load, round & 1, 1u << 16);
-        umma_commit(&s_mma[0]);
-        mbar_wait_bounded(&s_mma[0], 0, 1u << 16);
+        // a wait gave up: before the block's memory goes away, let the loads and MMAs still
+        // in flight land, each wait bounded and on a phase that nothing else has completed
+        if (!matrices) mbar_wait_bounded(&s_matrix, 0, kTmaWaitLimit);
+        if (loading) mbar_wait_bounded(&s_load, round & 1, kTmaWaitLimit);
+        umma_commit(&s_drain);
+        mbar_wait_bounded(&s_drain, 0, kTmaWaitLimit);
       }
     }
   } else {
@@ -430,7 +461,7 @@ __global__ void __launch_bounds__(kMmThreads, 1) k_ntt_pass_mm(F f, const NttPas
       }
       if (prescale) {
         // the coset factors g^pos, on the rows as they landed
-        if (!(ok = mm_wait(&s_load, round & 1, &s_failed))) break;
+        if (!(ok = mm_wait_warp(&s_load, round & 1, &s_failed))) break;
 #pragma unroll 1
         for (int i = tid; i < (1 << kMmTileLog); i += 32 * kMmWorkers) {
           const int64_t pos = o * B + (int64_t)(i >> lc) * S + j0c + (i & (C - 1));
@@ -465,7 +496,7 @@ __global__ void __launch_bounds__(kMmThreads, 1) k_ntt_pass_mm(F f, const NttPas
           fe_load(w, tw + 4 * ((k << l2) + j0));
           fe_load(v, tw + 4 * (((k + 8) << l2) + j0));
         }
-        if (!(ok = mm_wait(&s_mma[h], 0, &s_failed))) break;
+        if (!(ok = mm_wait_warp(&s_mma[h], 0, &s_failed))) break;
         tmem_fence_after();
         load_pair(s, d, k);
         mm_reduce(x, s, mp.mu, f);
@@ -473,7 +504,7 @@ __global__ void __launch_bounds__(kMmThreads, 1) k_ntt_pass_mm(F f, const NttPas
         fe_mul_open(x, x, w, f);
         fe_mul_open(y, y, v, f);
         // every MMA of the stage has read the tile before it changes
-        if (h == 0 && !(ok = mm_wait(&s_mma[1], 0, &s_failed))) break;
+        if (h == 0 && !(ok = mm_wait_warp(&s_mma[1], 0, &s_failed))) break;
         tile_store(rows, row1 + (k << lc), x);
         tile_store(rows, row1 + ((k + 8) << lc), y);
       }
@@ -521,7 +552,7 @@ __global__ void __launch_bounds__(kMmThreads, 1) k_ntt_pass_mm(F f, const NttPas
         bool hw, hv;
         uint64_t* px = pair ? target(m, k, w, hw) : target((block >> l2) * 128 + m, block & (r2 - 1), w, hw);
         uint64_t* py = pair ? target(m, k + 8, v, hv) : target(((block + 1) >> l2) * 128 + m, (block + 1) & (r2 - 1), v, hv);
-        if (!(ok = mm_wait(&s_mma[h], 1, &s_failed))) break;
+        if (!(ok = mm_wait_warp(&s_mma[h], 1, &s_failed))) break;
         tmem_fence_after();
         {
           uint32_t s[9], d[9];

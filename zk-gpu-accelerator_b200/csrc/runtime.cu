@@ -38,6 +38,7 @@ static Knob g_knobs[] = {
     {"ntt.batch_spin_limit", 0, 0, 1 << 30},  // polls before a batch tile's dependency wait gives up (0 = 2^22)
     {"ntt.tma", 1, 0, 1},                    // multi-pass transforms: TMA-fed persistent passes (1) or per-thread gathers (0)
     {"ntt.matrix", 1, 0, 1},                 // passes of 64..256 points as byte matrix products (1) or butterflies (0)
+    {"ntt.matrix_polls", 0, -1, 1 << 30},    // polls of a matrix pass's first wait before it gives up (0 = 2^24, -1 = none)
     {"ntt.lazy", 1, 0, 1},                   // TMA passes: values in [0, 2p) between butterfly rounds (p < 2^254)
     {"ntt.tma_grid", 1, 0, 1},               // TMA passes: one persistent wave (0) or one tile per block (1)
     {"ntt.tma_blocks_per_sm", 0, 0, 6},      // TMA passes of 128-thread blocks: registers capped for 5 or 6 blocks (0 = no cap)
