@@ -36,6 +36,10 @@ FIELDS = [
 BLS12_381_R = 0x73EDA753299D7D483339D80809A1D80553BDA402FFFE5BFEFFFFFFFF00000001
 
 
+def ints_rows(values) -> np.ndarray:
+    return np.array([[(v >> (64 * j)) & (2**64 - 1) for j in range(4)] for v in values], dtype=np.uint64)
+
+
 def rows_ints(t) -> list[int]:
     return wl.rows_to_ints(t.cpu().numpy())
 
@@ -526,3 +530,51 @@ def test_matrix_pass_waits_that_run_out_are_counted_and_leave_the_gpu_usable():
     out = subprocess.run([sys.executable, "-c", _WAITS_THAT_RUN_OUT], env=env, capture_output=True, text=True,
                          timeout=300)
     assert out.returncode == 0 and out.stdout.strip() == "ok", out.stderr
+
+
+@pytest.mark.parametrize("field", FIELDS)
+def test_rows_that_are_not_canonical_keep_their_residue_in_products(field):
+    """A row may hold any 256-bit value congruent to the element: a product by a canonical row and
+    the conversions give the canonical rows of its residue, at the top of the range (2^256 - p and
+    above) too; squaring such a row gives a row of the square's residue."""
+    import torch
+
+    p = field.modulus
+    r_inv = pow(1 << 256, -1, p)
+    rng = random.Random(p % 991)
+    tops = [2**256 - 1, 2**256 - 2, 2**256 - p, 2**256 - p - 1, 2**256 - p + 1, 2**255, 2**255 - 1, p, p + 1]
+    tops += [rng.randrange(2**256 - p, 2**256) for _ in range(200)] + [rng.randrange(2**256) for _ in range(200)]
+    b = [rng.randrange(p) for _ in tops]
+
+    def rows(values):
+        return torch.from_numpy(ints_rows(values)).cuda()
+
+    assert rows_ints(field.mul(rows(tops), rows(b))) == [x * y * r_inv % p for x, y in zip(tops, b)]
+    assert rows_ints(field.mul(rows(b), rows(tops))) == [x * y * r_inv % p for x, y in zip(tops, b)]
+    assert rows_ints(field.from_montgomery(rows(tops))) == [x * r_inv % p for x in tops]
+    assert rows_ints(field.to_montgomery(rows(tops))) == [(x << 256) % p for x in tops]
+    x = rows(tops)
+    assert [v % p for v in rows_ints(field.mul(x, x))] == [v * v * r_inv % p for v in tops]
+
+
+@pytest.mark.parametrize("log_n", [8, 12, 20])
+def test_coset_ntt_of_rows_that_are_not_canonical(log_n):
+    """A forward coset transform multiplies its rows first, so they may be any 256-bit values: the
+    same rows as their residues', through every form of the passes."""
+    import torch
+    from zkgpu import _native
+
+    n = 1 << log_n
+    plain = wl.uniform_fr(540 + log_n, n)
+    high = plain.copy()
+    high[:64] = ints_rows([v + (2**256 - 1 - v) // R * R for v in wl.rows_to_ints(plain[:64])])
+    assert min(wl.rows_to_ints(high[:64])) >= 2**256 - R
+    rows, high = torch.from_numpy(plain).cuda(), torch.from_numpy(high).cuda()
+    try:
+        for knob in ("ntt.matrix", "ntt.tma", None):  # each form off in turn
+            assert bool((BN254_FR.ntt(high, coset=5) == BN254_FR.ntt(rows, coset=5)).all()), knob
+            if knob:
+                _native.tune_set(knob, 0)
+    finally:
+        _native.tune_set("ntt.matrix", 1)
+        _native.tune_set("ntt.tma", 1)

@@ -405,7 +405,9 @@ struct CiosSum {
 // CIOS (coarsely integrated operand scanning): for each word b_i, t += a b_i,
 // then t = (t + m p) / 2^32 with m = t_0 (-p^-1) mod 2^32. Bounds: the sum stays
 // below 2^288 within a row (so O never carries out of its eight words and one word
-// `top` takes E's carries), and below 2^256 between rows, for a + p < 2^256.
+// `top` takes E's carries), and below 2^256 between rows, for a + p < 2^256. b may be
+// any 256-bit value, so a factor that may not be canonical goes second (or through
+// fe_fit).
 //
 // What bounds it: the 128 wide multiply-adds, each four cycles of a scheduler's
 // multiply pipe (32 lanes per SM per clock). Products kept on two fixed grids of
@@ -735,22 +737,22 @@ __device__ __forceinline__ void fe_dbl(uint32_t r[8], const uint32_t a[8], const
   fe_add(r, a, a, f);
 }
 
-// Montgomery form of a plain canonical value: a * R^2 * R^-1 = aR
+// Montgomery form of a plain value (any 256 bits): a * R^2 * R^-1 = aR
 // (zkgpu/field256_gpu.py:307-310).
 template <class F>
 __device__ __forceinline__ void fe_to_mont(uint32_t r[8], const uint32_t a[8], const F& f) {
   uint32_t r2[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) r2[j] = f.r2(j);
-  fe_mul(r, a, r2, f);
+  fe_mul(r, r2, a, f);
 }
 
-// Plain value of a Montgomery-form element: aR * 1 * R^-1 = a
+// Plain value of a Montgomery-form element (any 256 bits): aR * 1 * R^-1 = a
 // (zkgpu/field256_gpu.py:318-319).
 template <class F>
 __device__ __forceinline__ void fe_from_mont(uint32_t r[8], const uint32_t a[8], const F& f) {
   uint32_t one[8] = {1, 0, 0, 0, 0, 0, 0, 0};
-  fe_mul(r, a, one, f);
+  fe_mul(r, one, a, f);
 }
 
 // ---- inversion ----------------------------------------------------------------
@@ -933,6 +935,13 @@ __device__ __forceinline__ void fe_sub_p(uint32_t a[8], const F& f) {
       : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4]), "+r"(a[5]), "+r"(a[6]), "+r"(a[7])
       : "r"(f.p(0)), "r"(f.p(1)), "r"(f.p(2)), "r"(f.p(3)), "r"(f.p(4)), "r"(f.p(5)), "r"(f.p(6)),
         "r"(f.p(7)));
+}
+
+// a - p where a may be 2^256 - p or more (the top word tells; such an a is not below p,
+// as p < 2^255), else a: the same residue, fit for a first factor of fe_mul.
+template <class F>
+__device__ __forceinline__ void fe_fit(uint32_t a[8], const F& f) {
+  if (a[7] >= ~f.p(7)) fe_sub_p(a, f);
 }
 
 // Reduce any 256-bit value into [0, p) by repeated subtraction. For BN254

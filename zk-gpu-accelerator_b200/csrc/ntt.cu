@@ -498,7 +498,7 @@ __device__ __forceinline__ void ntt_tile(const F& f, const NttPass& a, int64_t b
         fe_load_nc(hi, a.g_hi + 4 * ((uint64_t)pos >> a.gs));
         ntt_mul<kShared>(lo, lo, hi, f);
       }
-      mul_l(x, x, lo);
+      mul_l(x, lo, x);
     }
     fe_store(sm + sm_index(c, jr, lr), x);
   }
@@ -801,7 +801,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_ntt_pass_tma(F f, cons
         fe_load_nc(hi2, a.g_hi + 4 * ((uint64_t)pos >> a.gs));
         fe_mul(g, g, hi2, f);
       }
-      bf_mul(x, x, g);
+      bf_mul(x, g, x);
     };
 
     // ---- decimation in frequency ----
@@ -1863,7 +1863,7 @@ __global__ void __launch_bounds__(128) k_ntt_cross(F f, const uint64_t* in, uint
         fe_load_nc(lo, st.g_lo + 4 * (j & gm));
         fe_load_nc(hi, st.g_hi + 4 * (j >> st.gs));
         fe_mul(lo, lo, hi, f);
-        fe_mul(a[j1], a[j1], lo, f);
+        fe_mul(a[j1], lo, a[j1], f);
       }
     }
 #pragma unroll

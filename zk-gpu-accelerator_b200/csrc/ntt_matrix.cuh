@@ -475,6 +475,7 @@ __global__ void __launch_bounds__(kMmThreads, 1) k_ntt_pass_mm(F f, const NttPas
             fe_load_nc(h, a.g_hi + 4 * ((uint64_t)pos >> a.gs));
             fe_mul(g, g, h, f);
           }
+          fe_fit(x, f);
           fe_mul_open(x, x, g, f);
           tile_store(rows, i, x);
         }

@@ -26,6 +26,7 @@ __global__ void __launch_bounds__(256) k_quotient_pointwise(const uint64_t* a, c
     fe_load_nc(x, a + 4 * i);
     fe_load_nc(y, b + 4 * i);
     fe_load_nc(w, c + 4 * i);
+    fe_fit(x, f);
     fe_mul(x, x, y, f);
     fe_sub(x, x, w, f);
     fe_mul(x, x, z, f);
