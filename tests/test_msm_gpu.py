@@ -400,6 +400,44 @@ def test_window_sums_that_equal_or_cancel_the_doubled_sum(window_size, sign):
                 assert got == want, (j, shift, last)
 
 
+@pytest.mark.parametrize("n, window_size", [(1 << 16, 1), (1 << 16, 4), (100_003, 6)])
+def test_few_buckets_of_many_runs_each(n, window_size):
+    """Small windows: every bucket owns hundreds to thousands of runs, which must go in chunks. The
+    same point as the default window's, and the merge (an addition for every eight or more of the
+    bucket kernel's) takes less time than the bucket kernel: one quad a bucket takes ten times as
+    long."""
+    bases = _bases(n, 381)
+    scalars = _native.torch_module().from_numpy(wl.uniform_fr(382, n)).cuda()
+    want = msm_pippenger_rows(bases, scalars)
+    assert msm_pippenger_rows(bases, scalars, window_size=window_size) == want
+    _native.profile_enable(True)
+    try:
+        msm_pippenger_rows(bases, scalars, window_size=window_size)
+        spans = _native.profile_report()
+    finally:
+        _native.profile_enable(False)
+    assert spans["msm_acc_merge"][1] < spans["msm_acc_points"][1], spans
+
+
+def test_a_table_of_few_buckets():
+    """A table at the smallest window: 128 buckets of some 4,000 runs each."""
+    from zkgpu.msm_gpu import FixedBaseTable
+
+    n = 1 << 17
+    bases = _bases(n, 391)
+    scalars = _native.torch_module().from_numpy(wl.uniform_fr(392, n)).cuda()
+    want = msm_pippenger_rows(bases, scalars)
+    table = FixedBaseTable(bases, 8)
+    assert table.msm(scalars) == want
+    _native.profile_enable(True)
+    try:
+        table.msm(scalars)
+        spans = _native.profile_report()
+    finally:
+        _native.profile_enable(False)
+    assert spans["msm_acc_merge"][1] < spans["msm_acc_points"][1], spans
+
+
 # ------------------------------------------------------------------
 # Bucket runs whose products reduce on the tensor cores (the default) against the ones with
 # every product in place (msm.call_products = 0)

@@ -1695,6 +1695,24 @@ static int first_level_log(int64_t windows, int64_t nb, int cap) {
   return l;
 }
 
+// The most runs of a bucket that one quad adds one after another (k_msm_merge); a bucket
+// of more goes in chunks of `chunk` runs, a block each. 32, or twice the average (so that
+// uniform scalars make no chunks) where the quads add their `runs` / `keys` runs sooner
+// than the blocks would: counted in dependent additions, a wave of 148 x 4 blocks at a
+// time, 32 quads of average length against one chunk a block (runs / 32 and a tree).
+// Measured on B200, all merge launches with quads and with blocks (ms), * what this takes:
+// one MSM of 2^20 points, window 4 24.0 and 1.06*, 10 0.76 and 0.67*, 11 0.39* and 0.96,
+// 12 0.34* and 1.22; 2^18, window 9 0.85 and 0.86*; 2^16, window 4 5.6 and 0.30*; a table of
+// 2^20 points, window 8 10.8 and 0.29*, 12 1.79 and 0.65*, 13 0.60 and 0.44*, 14 0.33* and
+// 0.69.
+static int64_t merge_threshold(int64_t runs, int64_t keys, int64_t chunk) {
+  const int64_t average = runs / std::max<int64_t>(1, keys), wave = 148 * 4;
+  const int64_t chunks = keys * ((average + chunk - 1) / chunk);
+  const int64_t quads = average * ((keys + 32 * wave - 1) / (32 * wave));
+  const int64_t blocks = (std::min(average, chunk) / 32 + 6) * ((chunks + wave - 1) / wave);
+  return average <= 16 || blocks < quads ? 32 : 2 * average;
+}
+
 // The longest automatic run of sorted pairs in a one-MSM call, twice
 // "msm.call_pairs_cap" (default 16; batches go up to 64). A bucket block then lasts
 // about 0.3 ms at 2^22 points, so kernels the caller runs beside the MSM on other
@@ -1763,11 +1781,11 @@ static int make_plan(const int64_t* sizes, int count, int w, MsmPlan& p, int tab
   p.red_l = first_level_log(p.windows, p.nb, p.log_l);
   p.call_products = tune_get("msm.call_products");
   p.T1 = (p.E_list + p.k1 - 1) / p.k1;
-  // A bucket of at most 32 runs, or twice the average (uniform scalars), is one
-  // quad's; larger ones go in chunks of 32 k2 runs, at most one per thr and one per
-  // 32 k2 runs of the T1 (a run belongs to two buckets at most).
+  // A bucket of at most merge_thr runs is one quad's; larger ones go in chunks of 32 k2
+  // runs, at most one per merge_thr and one per 32 k2 runs of the T1 (a run belongs to two
+  // buckets at most).
   const int64_t chunk = 32 * (int64_t)p.k2;
-  p.merge_thr = (uint32_t)std::max<int64_t>(32, 2 * (p.T1 / std::max<int64_t>(1, keys_used)));
+  p.merge_thr = (uint32_t)merge_threshold(p.T1, keys_used, chunk);
   p.max_chunks = p.T1 <= p.merge_thr ? 0 : 2 * p.T1 / p.merge_thr + 2 * p.T1 / chunk + 1;
   // CUB's temporary storage for sorting E pairs (a size query; launches nothing)
   cub::DoubleBuffer<uint32_t> kb(nullptr, nullptr), vb(nullptr, nullptr);
