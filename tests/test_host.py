@@ -316,6 +316,27 @@ def test_product_never_imports_the_oracle():
 # ------------------------------------------------------------------
 
 
+def test_a_table_measured_with_other_kernels_is_not_reused(tmp_path, monkeypatch):
+    """A table stored under a key without the kernels' revision (or with another one) was measured
+    with kernels that are gone."""
+    from types import SimpleNamespace
+
+    from zkgpu import autotune
+
+    props = SimpleNamespace(name="NVIDIA B200", major=10, minor=0, multi_processor_count=148)
+    cuda = SimpleNamespace(current_device=lambda: 0, get_device_properties=lambda i: props)
+    monkeypatch.setattr(_native, "require_cuda", lambda: SimpleNamespace(cuda=cuda))
+    abi = _native.lib().zkb_version()
+    old = f"NVIDIA B200|sm_100|148 SMs|abi {abi}"
+    entry = {"msm": {22: {"window": 9}}, "ntt": {}}
+    path = autotune.save({"device": old, **entry}, tmp_path / "tune.json")
+    assert autotune.load(path) is None
+    path = autotune.save({"device": autotune.device_key(), **entry}, path)
+    assert autotune.load(path)["msm"]["22"]["window"] == 9
+    monkeypatch.setattr(autotune, "KERNELS", autotune.KERNELS + 1)
+    assert autotune.load(path) is None
+
+
 def test_per_size_tables_drive_the_plans(tmp_path):
     from zkgpu import autotune
 

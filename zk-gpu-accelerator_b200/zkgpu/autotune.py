@@ -17,7 +17,8 @@ A choice changes only speed: every candidate computes the same rows and
 points (the GPU tests check the NTT plans and windows against the
 reference). The table is saved as JSON (default ~/.cache/zkgpu/tune.json,
 or $ZKGPU_TUNE_CACHE) under a key naming the GPU, its compute capability and
-the library's ABI version, and autotune() reuses it when the key matches.
+the library's ABI version and kernels, and autotune() reuses it when the key
+matches.
 """
 
 from __future__ import annotations
@@ -33,6 +34,9 @@ from zkgpu import _native
 CACHE_ENV = "ZKGPU_TUNE_CACHE"
 NTT_KEYS = ("ntt.max_log_radix", "ntt.cta_log_elems", "ntt.threads")
 MSM_KEY = "msm.window"
+# Raised when kernels change so that choices measured before no longer hold (1: butterfly NTT passes
+# alone, merge levels; 2: matrix NTT passes, quads in the MSM's merge and reduction).
+KERNELS = 2
 
 
 def default_cache_path() -> Path:
@@ -42,7 +46,7 @@ def default_cache_path() -> Path:
 def device_key() -> str:
     torch = _native.require_cuda()
     p = torch.cuda.get_device_properties(torch.cuda.current_device())
-    return f"{p.name}|sm_{p.major}{p.minor}|{p.multi_processor_count} SMs|abi {_native.lib().zkb_version()}"
+    return f"{p.name}|sm_{p.major}{p.minor}|{p.multi_processor_count} SMs|abi {_native.lib().zkb_version()}|kernels {KERNELS}"
 
 
 def _median_ms(fn, reps: int) -> float:
