@@ -366,7 +366,7 @@ int zkb_msm_fixed_batch(const zkb_msm_job* jobs, int count, void* workspace, siz
  * every operation; the same rows either way), "ntt.matrix" (1: transforms of
  * 2^20 to 2^24 rows over BN254's Fr run passes of 64 to 256 points as byte matrix
  * products on the tensor cores, while the knobs of the butterfly passes are at their
- * defaults; 0: butterfly passes; the same rows either way), "ntt.matrix_polls"
+ * defaults and the size has no per-size tile or block size; 0: butterfly passes; the same rows either way), "ntt.matrix_polls"
  * (polls of such a pass's first wait, for its matrices, before it gives up, its
  * block stops early and zkb_ntt_wait_timeouts counts it; 0 = the default 2^24, as
  * for every other wait, -1 = none at all);

@@ -516,6 +516,40 @@ print("ok")
 """
 
 
+_TILES_ASKED_FOR = """
+import torch
+from zkgpu import _native, workloads as wl
+from zkgpu.field256_gpu import BN254_FR
+
+lib = _native.lib()
+rows = BN254_FR.to_montgomery(wl.uniform_fr(521, 1 << 20))
+want = BN254_FR.ntt(rows)
+_native.tune_set("ntt.matrix_polls", -1)  # a matrix pass would give up and be counted
+for key, value in (("ntt.cta_log_elems", 11), ("ntt.threads", 256)):
+    for ask, none in ((_native.tune_set, (key, 0)), (lambda k, v: _native.tune_set_sized(k, 20, v), (key, 0))):
+        ask(key, value)
+        assert bool((BN254_FR.ntt(rows) == want).all()), key
+        ask(*none)
+assert lib.zkb_ntt_wait_timeouts() == 0
+print("ok")
+"""
+
+
+def test_a_tile_or_block_size_asked_for_is_honoured_from_either_table():
+    """A process-wide knob and a per-size entry of the same name have the same effect: both ask for
+    butterfly passes of that shape where matrix passes would run (in a process of its own, as the
+    next test)."""
+    import subprocess
+    import sys
+
+    from conftest import ROOT
+
+    env = {**os.environ, "PYTHONPATH": str(ROOT / "zk-gpu-accelerator_b200")}
+    out = subprocess.run([sys.executable, "-c", _TILES_ASKED_FOR], env=env, capture_output=True, text=True,
+                         timeout=300)
+    assert out.returncode == 0 and out.stdout.strip() == "ok", out.stderr
+
+
 def test_matrix_pass_waits_that_run_out_are_counted_and_leave_the_gpu_usable():
     """With no polls ("ntt.matrix_polls" = -1) the control lane's first wait gives up at once and the
     worker warps' waits follow: each block counts itself once, lets its loads land and returns; the

@@ -337,6 +337,18 @@ def test_a_table_measured_with_other_kernels_is_not_reused(tmp_path, monkeypatch
     assert autotune.load(path) is None
 
 
+def test_autotuner_measures_the_matrix_passes_once():
+    """From 2^20 rows the library's own plan (matrix passes) is one candidate among the butterfly
+    plans; below, where it is a butterfly plan too, there is none."""
+    from zkgpu import autotune
+
+    for lg in range(10, 25):
+        cands = autotune._ntt_candidates(lg)
+        assert len(set(cands)) == len(cands)
+        assert cands.count((0, 0, 0)) == (1 if lg >= 20 else 0), lg
+        assert all(0 not in c for c in cands if c != (0, 0, 0)), lg
+
+
 def test_per_size_tables_drive_the_plans(tmp_path):
     from zkgpu import autotune
 

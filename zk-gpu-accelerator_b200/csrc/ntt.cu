@@ -1412,6 +1412,17 @@ struct PassLaunch {
   size_t smem;
 };
 
+// The tile (log2 rows) and block size asked for at 2^log_n rows, 0 for none: a per-size
+// table entry takes precedence over the knob.
+static int asked_tile(int log_n) {
+  const int v = tune_get_sized("ntt.cta_log_elems", log_n);
+  return v ? v : tune_get("ntt.cta_log_elems");
+}
+static int asked_threads(int log_n) {
+  const int v = tune_get_sized("ntt.threads", log_n);
+  return v ? v : tune_get("ntt.threads");
+}
+
 // The passes of one transform. cta_log / threads: the tile and block size,
 // or 0 for the size-based choice (and the "ntt.cta_log_elems" / "ntt.threads"
 // knobs, which override it). batch: the transform is part of a batch launch
@@ -1428,16 +1439,13 @@ static void plan_passes(int64_t n, int log_n, int invert, const RootTables& rt,
   // CTA's loads and barriers overlap another's products; measured on B200
   // against 1024-row tiles of 256 threads (and 4096-row tiles of 512 threads
   // from 2^24): 18-27 % faster from 2^11 to 2^16 rows, within 2 % at 2^17-2^18.
-  // A per-size table entry takes precedence over the knob, which takes
-  // precedence over the rule.
+  // What is asked for takes precedence over the rule.
   if (cta_log == 0) {
-    cta_log = tune_get_sized("ntt.cta_log_elems", log_n);
-    if (cta_log < 9) cta_log = tune_get("ntt.cta_log_elems");
+    cta_log = asked_tile(log_n);
     if (cta_log < 9) cta_log = 9;
   }
   if (threads == 0) {
-    threads = tune_get_sized("ntt.threads", log_n);
-    if (threads < 64) threads = tune_get("ntt.threads");
+    threads = asked_threads(log_n);
     if (threads < 64) threads = 0;  // by each pass's tile, below
   }
   passes.clear();
@@ -1562,14 +1570,15 @@ static int launch_pass_tma(const F& f, const PassLaunch& L, int64_t n, int P, in
 // Whether a transform's passes go through k_ntt_pass_mm ("ntt.matrix", default 1):
 // BN254 Fr with the library's tables, every pass of 64, 128 or 256 points on whole
 // 2048-row tiles, at least two tiles for each SM (the blocks are persistent and load
-// 128 KiB of matrices first), and none of the butterfly passes' own knobs set.
+// 128 KiB of matrices first), and nothing asked for that only butterfly passes have: none of
+// their own knobs set, no tile or block size for this transform's size.
 // Measured on B200, butterfly against matrix passes: 2^20 rows 0.231 / 0.198 ms, 2^22
 // 0.898 / 0.623; 2^19 rows are 256 tiles for 148 SMs, two rounds of which the second
 // is three quarters full.
 static bool matrix_passes(const RootTables& rt, const std::vector<PassLaunch>& passes, int64_t n, int sms) {
   if (!rt.mm[0] || tune_get("ntt.matrix") == 0 || (n >> kMmTileLog) < 2 * sms) return false;
   if (tune_get("ntt.tma_grid") != 1 || tune_get("ntt.tma_blocks_per_sm") != 0 || tune_get("ntt.lazy") == 0 ||
-      tune_get("ntt.cta_log_elems") != 0 || tune_get("ntt.threads") != 0) {
+      asked_tile(passes[0].a.log_n) != 0 || asked_threads(passes[0].a.log_n) != 0) {
     return false;
   }
   for (const PassLaunch& L : passes) {

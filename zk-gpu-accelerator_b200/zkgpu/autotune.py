@@ -11,7 +11,9 @@ which every later call, batched or not, plans with:
 
   msm.window                      the default window of an MSM of 2^log points
   ntt.max_log_radix / ntt.cta_log_elems / ntt.threads
-                                  the pass split, tile and block of an NTT of 2^log rows
+                                  the pass split, tile and block of an NTT of 2^log rows,
+                                  or all 0: the library's own plan, which from 2^20 rows
+                                  has matrix passes instead of tiles and blocks to choose
 
 A choice changes only speed: every candidate computes the same rows and
 points (the GPU tests check the NTT plans and windows against the
@@ -112,7 +114,8 @@ def tune_msm(log_sizes, *, reps: int = 3, spread: int = 2, seed: int = 1) -> dic
 
 
 def _ntt_candidates(lg: int) -> list[tuple[int, int, int]]:
-    cands = []
+    # a tile or block size asks for butterfly passes, so the matrix passes are a candidate of their own
+    cands = [(0, 0, 0)] if lg >= 20 else []
     for radix in (12, 11, 10, 8):
         if radix < 12 and (lg + radix - 1) // radix == (lg + 11) // 12:
             continue  # the same number of passes as 12-bit ones: same plan
