@@ -335,9 +335,10 @@ int zkb_msm_fixed_batch(const zkb_msm_job* jobs, int count, void* workspace, siz
  * the workspace size queries): "msm.pairs_per_thread" (sorted pairs a bucket
  * thread adds in turn, 8..4096; default 0 = by size: the pair bound over 2^19,
  * as a power of two within 8..64, or within 8..32 for zkb_msm and
- * zkb_msm_no_alloc), "msm.call_pairs_cap" (16: half that upper limit for the
- * one-MSM calls, 8..64; shorter bucket blocks let work on other streams reach
- * the SMs sooner), "msm.slots_per_thread" (8: runs a quad of lanes adds of a
+ * zkb_msm_no_alloc), "msm.call_pairs_cap" (8..64: that upper limit for the
+ * one-MSM calls once it is set; never set, it reads 16 and the limit is 32.
+ * Shorter bucket blocks let work on other streams reach the SMs sooner),
+ * "msm.slots_per_thread" (8: runs a quad of lanes adds of a
  * bucket's merge chunk, 256 a block), "msm.reduce_log_segment" (4: the first
  * reduction level sums 16 buckets a quad of lanes, 512 a block), "msm.sort" (1:
  * pairs grouped by a counting sort that skips zero digits; 0: a radix sort

@@ -400,6 +400,20 @@ def test_window_sums_that_equal_or_cancel_the_doubled_sum(window_size, sign):
                 assert got == want, (j, shift, last)
 
 
+@pytest.mark.parametrize("n", [1 << 18, 1 << 20, 1 << 22])
+@pytest.mark.parametrize("cap", [8, 16, 32, 64])
+def test_the_run_cap_of_a_one_msm_call_is_the_length_asked_for(n, cap):
+    """ "msm.call_pairs_cap" bounds the automatic run length (pairs over 2^19, a power of two from 8
+    up) at the value set: the workspace is the one of runs of that length."""
+    lib = _native.lib()
+    pairs = 16 * n  # 2 W n at the default window, 16
+    want = 8
+    while want < cap and want << 20 <= pairs:
+        want *= 2
+    with_cap = _with_knobs({"msm.call_pairs_cap": cap}, lambda: lib.zkb_msm_workspace_bytes(n, 16))
+    assert with_cap == _with_knobs({"msm.pairs_per_thread": want}, lambda: lib.zkb_msm_workspace_bytes(n, 16)) > 0
+
+
 @pytest.mark.parametrize("n, window_size", [(1 << 16, 1), (1 << 16, 4), (100_003, 6)])
 def test_few_buckets_of_many_runs_each(n, window_size):
     """Small windows: every bucket owns hundreds to thousands of runs, which must go in chunks. The

@@ -39,6 +39,7 @@ void count_launch();
 
 // Tuning knobs read when a call plans its work (zkb_tune_set / zkb_tune_get).
 int tune_get(const char* key);
+bool tune_is_set(const char* key);  // by zkb_tune_set, to any value
 
 // Per-size tuning tables (zkb_tune_set_sized): the entry for log2 size log_n,
 // or 0 when the table has none.

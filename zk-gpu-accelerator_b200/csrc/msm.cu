@@ -1713,15 +1713,15 @@ static int64_t merge_threshold(int64_t runs, int64_t keys, int64_t chunk) {
   return average <= 16 || blocks < quads ? 32 : 2 * average;
 }
 
-// The longest automatic run of sorted pairs in a one-MSM call, twice
-// "msm.call_pairs_cap" (default 16; batches go up to 64). A bucket block then lasts
-// about 0.3 ms at 2^22 points, so kernels the caller runs beside the MSM on other
-// streams (a transform of higher priority) wait at most that long for an SM at each of
-// their launches; the knob's value was the run itself when an addition took twice as
-// long. Longer runs leave fewer of them to
-// merge: at 2^22 points runs of 32 take the merge from 1.28 to 0.66 ms against 16, the
-// bucket kernel the same, on B200.
-static int single_call_pairs_cap() { return 2 * tune_get("msm.call_pairs_cap"); }
+// The longest automatic run of sorted pairs in a one-MSM call: "msm.call_pairs_cap" once
+// the caller has set it, else 32 (batches go up to 64). A bucket block of 32 lasts about
+// 0.3 ms at 2^22 points, so kernels the caller runs beside the MSM on other streams (a
+// transform of higher priority) wait at most that long for an SM at each of their
+// launches. Shorter runs leave more of them to merge: at 2^22 points 1.28 ms with 16, 0.66
+// with 32, the bucket kernel the same, on B200.
+static int single_call_pairs_cap() {
+  return tune_is_set("msm.call_pairs_cap") ? tune_get("msm.call_pairs_cap") : 32;
+}
 
 // Plan for a batch of jobs with point counts sizes[0..count) at window w.
 static int make_plan(const int64_t* sizes, int count, int w, MsmPlan& p, int table = 0, int k1 = 0,

@@ -20,12 +20,13 @@ void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 struct Knob {
   const char* name;
   int value, lo, hi;
+  bool set = false;  // by zkb_tune_set
 };
 static Knob g_knobs[] = {
     {"msm.pairs_per_thread", 0, 0, 4096},    // sorted pairs each bucket thread adds (8..4096; 0 = by size)
     {"msm.slots_per_thread", 8, 4, 4096},    // runs a quad adds of a large bucket's chunk
     {"msm.reduce_log_segment", 4, 0, 8},     // log2 of the buckets a quad sums in the first reduction level
-    {"msm.call_pairs_cap", 16, 8, 64},       // half the longest automatic bucket run of a one-MSM call
+    {"msm.call_pairs_cap", 16, 8, 64},       // once set: the longest automatic bucket run of a one-MSM call
     {"msm.call_products", 1, 0, 1},          // bucket kernels' default products (1) or all of them in place (0)
     {"msm.sort", 1, 0, 1},                   // pairs grouped by a counting sort (1) or a radix sort (0)
     {"msm.affine_rounds", 0, -1, 8},         // affine rounds before the XYZZ levels (0 = none, -1 = by size)
@@ -60,6 +61,12 @@ int tune_get(const char* key) {
   std::lock_guard<std::mutex> lock(g_knob_mutex);
   Knob* k = find_knob(key);
   return k ? k->value : 0;
+}
+
+bool tune_is_set(const char* key) {
+  std::lock_guard<std::mutex> lock(g_knob_mutex);
+  const Knob* k = find_knob(key);
+  return k && k->set;
 }
 
 // ---- per-size tuning tables ---------------------------------------------------
@@ -255,6 +262,7 @@ int zkb_tune_set(const char* key, int value) {
     return zkb::fail(ZKB_EINVAL, "%s must be in %d..%d, got %d", k->name, k->lo, k->hi, value);
   }
   k->value = value;
+  k->set = true;
   return ZKB_OK;
 }
 
