@@ -492,6 +492,39 @@ def test_matrix_passes_equal_butterfly_passes(log_n, table_mb):
     assert lib.zkb_ntt_wait_timeouts() == 0
 
 
+def _run_alone(program: str) -> None:
+    """Runs *program* in a process of its own: what the library counts and caches starts empty there."""
+    import subprocess
+    import sys
+
+    from conftest import ROOT
+
+    env = {**os.environ, "PYTHONPATH": str(ROOT / "zk-gpu-accelerator_b200")}
+    out = subprocess.run([sys.executable, "-c", program], env=env, capture_output=True, text=True, timeout=300)
+    assert out.returncode == 0 and out.stdout.strip() == "ok", out.stderr
+
+
+_COSET_TABLE_WITHOUT_MATRICES = """
+from zkgpu import _native, workloads as wl
+from zkgpu.field256_gpu import BN254_FR
+
+rows = BN254_FR.to_montgomery(wl.uniform_fr(522, 1 << 20))
+_native.tune_set("ntt.full_table_mb", 32)  # the 2^20 factors of 32 bytes, not the matrices beside them
+got = BN254_FR.ntt(rows, coset=5)
+for knob in ("ntt.matrix", "ntt.tma"):
+    _native.tune_set(knob, 0)
+    assert bool((got == BN254_FR.ntt(rows, coset=5)).all()), knob
+assert _native.lib().zkb_ntt_wait_timeouts() == 0
+print("ok")
+"""
+
+
+def test_matrix_passes_scale_by_a_full_coset_table_without_matrices():
+    """A budget that holds a coset's n factors but not its matrices: the first matrix pass multiplies
+    its rows by the table as they land."""
+    _run_alone(_COSET_TABLE_WITHOUT_MATRICES)
+
+
 _WAITS_THAT_RUN_OUT = """
 import torch
 from zkgpu import _native, workloads as wl
@@ -539,15 +572,7 @@ def test_a_tile_or_block_size_asked_for_is_honoured_from_either_table():
     """A process-wide knob and a per-size entry of the same name have the same effect: both ask for
     butterfly passes of that shape where matrix passes would run (in a process of its own, as the
     next test)."""
-    import subprocess
-    import sys
-
-    from conftest import ROOT
-
-    env = {**os.environ, "PYTHONPATH": str(ROOT / "zk-gpu-accelerator_b200")}
-    out = subprocess.run([sys.executable, "-c", _TILES_ASKED_FOR], env=env, capture_output=True, text=True,
-                         timeout=300)
-    assert out.returncode == 0 and out.stdout.strip() == "ok", out.stderr
+    _run_alone(_TILES_ASKED_FOR)
 
 
 def test_matrix_pass_waits_that_run_out_are_counted_and_leave_the_gpu_usable():
@@ -555,15 +580,7 @@ def test_matrix_pass_waits_that_run_out_are_counted_and_leave_the_gpu_usable():
     worker warps' waits follow: each block counts itself once, lets its loads land and returns; the
     next transform is exact again.
     In a process of its own: the count is the library's and other tests want it to be 0."""
-    import subprocess
-    import sys
-
-    from conftest import ROOT
-
-    env = {**os.environ, "PYTHONPATH": str(ROOT / "zk-gpu-accelerator_b200")}
-    out = subprocess.run([sys.executable, "-c", _WAITS_THAT_RUN_OUT], env=env, capture_output=True, text=True,
-                         timeout=300)
-    assert out.returncode == 0 and out.stdout.strip() == "ok", out.stderr
+    _run_alone(_WAITS_THAT_RUN_OUT)
 
 
 @pytest.mark.parametrize("field", FIELDS)
