@@ -398,14 +398,15 @@ int zkb_tune_set_sized(const char* key, int log_n, int value);
 int zkb_tune_get_sized(const char* key, int log_n, int* value);
 
 /* Measured issue rates on the current device: loops of independent
- * mad.lo.u32, of mad.wide.u32 (32 x 32 -> 64-bit multiply-add) and of this
- * library's 256-bit Montgomery product over BN254's base field, each one
- * launch of as many 256-thread blocks as fit the SMs at once. *_per_clk_sm is
+ * mad.lo.u32, of wide multiply-adds (mad.wide.u32: 32 x 32 + 64 bits, in the
+ * carry chains that the products are made of) and of this library's 256-bit
+ * Montgomery product over BN254's base field, each one launch of as many
+ * 256-thread blocks as fit the SMs at once. *_per_clk_sm is
  * operations per SM per SM clock (from the SMs' cycle counters, independent
  * of the clock), *_per_s per second over the whole GPU (CUDA events), *_mhz
  * the SM clock that the two imply. They are the measured denominators of the
- * integer rooflines; the IMAD pipe peak at clock f is sms * madlo_per_clk_sm
- * * f. Takes a few tens of milliseconds and synchronises the stream. */
+ * integer rooflines; the peak at clock f is sms * f times the one per clock and
+ * SM. Takes a few tens of milliseconds and synchronises the stream. */
 typedef struct zkb_int_peaks {
   double madlo_per_clk_sm, madlo_per_s, madlo_mhz;
   double madwide_per_clk_sm, madwide_per_s, madwide_mhz;

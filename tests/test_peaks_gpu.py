@@ -29,3 +29,12 @@ def test_measured_integer_rates_are_plausible():
     assert 0.05 < p["montmul_per_clk_sm"] < p["madwide_per_clk_sm"] / 128 * 1.2, p
     for key in ("madlo_mhz", "madwide_mhz", "montmul_mhz"):
         assert 300.0 < p[key] < 2500.0, (key, p)
+
+
+def test_the_wide_multiply_rate_is_the_pipe_the_product_runs_on():
+    """The Montgomery product is 128 wide multiply-adds and little else, so it uses most of the rate
+    measured for them (a loop whose product is invariant reads three times as much); the low half
+    alone issues faster."""
+    p = _native.measure_int_peaks()
+    assert 0.7 < 128 * p["montmul_per_clk_sm"] / p["madwide_per_clk_sm"] < 1.2, p
+    assert p["madwide_per_clk_sm"] < 0.6 * p["madlo_per_clk_sm"], p
