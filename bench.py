@@ -123,7 +123,8 @@ IMAD_PER_SQR = 2 * 36 + IMAD_PER_FOLD     # a*a (each cross product once)
 IMAD_PER_MADD = 8 * IMAD_PER_MULMOD - IMAD_PER_FOLD + 2 * IMAD_PER_SQR
 # a scalar-field product of the transforms: a*b and 56 for the reduction (csrc/field.cuh)
 IMAD_PER_NTT_PRODUCT = 2 * (64 + 56)
-NTT_MATRIX_MIN_LOG = 20  # transforms from 2^20 rows run as byte matrix products (csrc/ntt_matrix.cuh)
+NTT_MATRIX_MIN_LOG = 20  # transforms from 2^20 rows run as byte matrix products (csrc/ntt_matrix.cuh),
+NTT_MATRIX_MAX_RADIX = 8  # where every pass has at most 2^8 points
 PRODUCTS_PER_MADD = 10
 
 
@@ -153,12 +154,24 @@ def ntt_products(n: int, log_n: int, passes: int | None = None) -> int:
     return int(per_row * n)
 
 
+def ntt_is_matrix(log_n: int, passes: int) -> bool:
+    """Whether the passes of a transform of 2^log_n rows are byte matrix products, as the library
+    chooses with the knobs as they are."""
+    from zkgpu import _native
+
+    as_matrix = _native.tune_get("ntt.matrix") and _native.tune_get("ntt.tma") and _native.tune_get("ntt.lazy")
+    asked = any(_native.tune_get(k) for k in ("ntt.cta_log_elems", "ntt.threads", "ntt.tma_blocks_per_sm"))
+    asked = asked or _native.tune_get("ntt.tma_grid") != 1
+    asked = asked or any(_native.tune_get_sized(k, log_n) for k in ("ntt.cta_log_elems", "ntt.threads"))
+    return bool(as_matrix) and not asked and NTT_MATRIX_MIN_LOG <= log_n <= NTT_MATRIX_MAX_RADIX * passes
+
+
 def ntt_imads(n: int, log_n: int, passes: int) -> tuple[int, int]:
     """(products, 32-bit multiply-adds) of one forward NTT as csrc/ntt.cu runs it. Matrix passes
     (csrc/ntt_matrix.cuh) multiply each row by an internal twiddle in every pass and by a boundary
     twiddle in all but the last, and reduce two matrix sums a row and pass (9 wide multiply-adds
     each); the sums themselves are on the tensor cores."""
-    if log_n < NTT_MATRIX_MIN_LOG:
+    if not ntt_is_matrix(log_n, passes):
         products = ntt_products(n, log_n, passes)
         return products, products * IMAD_PER_NTT_PRODUCT
     products = n * (2 * passes - 1)
@@ -563,16 +576,17 @@ def run_ours(args, rank: int, world: int, local_rank: int) -> dict | None:
         }
 
     measured = _native.measure_int_peaks()
-    imad_meas_t = measured["madlo_per_clk_sm"] * sm_count * mhz * 1e6 / 1e12
+    # the work is counted as two IMAD a wide multiply-add, so that is the rate to divide by
+    imad_meas_t = 2 * measured["madwide_per_clk_sm"] * sm_count * mhz * 1e6 / 1e12
     prod_meas = measured["montmul_per_clk_sm"] * sm_count * mhz * 1e6  # Montgomery products / s
     peak_measured = {
         "imad_t_per_s": round(imad_meas_t, 3), "montmul_per_s": round(prod_meas / 1e9, 3),
         "unit": "T IMAD/s; G products/s", "at_mhz": mhz,
         "per_clk_sm": {k: round(measured[f"{k}_per_clk_sm"], 3) for k in ("madlo", "madwide", "montmul")},
         "probe_mhz": {k: round(measured[f"{k}_mhz"], 1) for k in ("madlo", "madwide", "montmul")},
-        "source": "zkb_measure_int_peaks (csrc/peak.cu): one-wave loops of independent mad.lo.u32, "
-                  "mad.wide.u32 and 256-bit Montgomery products, SM cycle counters; scaled to the clock "
-                  "sampled in the timed region"}
+        "source": "zkb_measure_int_peaks (csrc/peak.cu): one-wave loops of independent mad.lo.u32, wide "
+                  "multiply-adds (the peak: two IMAD each) and 256-bit Montgomery products, SM cycle counters; "
+                  "scaled to the clock sampled in the timed region"}
 
     traffic_u = _profile_traffic("k_msm_acc_points_tc", step.n)
     traffic_s = _profile_traffic("k_msm_acc_points_tc_skewed", step.n)

@@ -104,6 +104,35 @@ def test_ntt_product_count_follows_the_pass_plan():
     assert bench.ntt_products(1 << 9, 9) == int(((0.25 + 3) + 0.5) * (1 << 9))  # one pass, odd radix
 
 
+def test_ntt_multiply_count_follows_the_librarys_choice_of_passes():
+    """Matrix passes' multiply-adds where the library runs them (2^20 to 2^24 rows in passes of at
+    most 2^8 points, nothing asked for that only butterfly passes have), else the butterflies'."""
+    from zkgpu import _native
+
+    def matrix(log_n, passes=3):
+        n = 1 << log_n
+        products, imads = bench.ntt_imads(n, log_n, passes)
+        butterflies = bench.ntt_products(n, log_n, passes)
+        assert (products, imads) == (butterflies, butterflies * bench.IMAD_PER_NTT_PRODUCT) or products == 5 * n
+        return products == 5 * n
+
+    assert [matrix(e) for e in (19, 20, 24, 25, 26)] == [False, True, True, False, False]
+    assert not matrix(20, 2)
+    for knob, value in (("ntt.matrix", 0), ("ntt.tma", 0), ("ntt.threads", 256), ("ntt.tma_grid", 0)):
+        default = _native.tune_get(knob)
+        try:
+            _native.tune_set(knob, value)
+            assert not matrix(22), knob
+        finally:
+            _native.tune_set(knob, default)
+    try:
+        _native.tune_set_sized("ntt.cta_log_elems", 22, 10)
+        assert not matrix(22) and matrix(23)
+    finally:
+        _native.tune_set_sized("ntt.cta_log_elems", 22, 0)
+    assert matrix(22)
+
+
 def test_gpus_flag_starts_one_rank_per_gpu_without_a_launcher():
     """`bench.py --gpus 2` with no torchrun environment starts two ranks itself; rank 0
     prints the line and sees both ranks (gloo here, NCCL on GPUs)."""
