@@ -414,6 +414,17 @@ def test_the_run_cap_of_a_one_msm_call_is_the_length_asked_for(n, cap):
     assert with_cap == _with_knobs({"msm.pairs_per_thread": want}, lambda: lib.zkb_msm_workspace_bytes(n, 16)) > 0
 
 
+@pytest.mark.parametrize("log_n, run", [(16, 8), (20, 16), (22, 32)])
+def test_the_workspace_is_what_the_kernels_write(log_n, run):
+    """Two key and two value arrays, the phi points, the buckets and two partial sums a run; the
+    rest (the sort's scratch, chunk lists, reduction pairs, counts) is a few percent."""
+    n, w = 1 << log_n, 16
+    windows, pairs = 8, 16 * n
+    large = 16 * pairs + 64 * n + 128 * windows * 2 ** (w - 1) + 256 * (-(-pairs // run))
+    total = _with_knobs({"msm.pairs_per_thread": run}, lambda: _native.lib().zkb_msm_workspace_bytes(n, w))
+    assert large < total < 1.07 * large
+
+
 @pytest.mark.parametrize("n, window_size", [(1 << 16, 1), (1 << 16, 4), (100_003, 6)])
 def test_few_buckets_of_many_runs_each(n, window_size):
     """Small windows: every bucket owns hundreds to thousands of runs, which must go in chunks. The

@@ -1822,14 +1822,12 @@ static int make_plan(const int64_t* sizes, int count, int w, MsmPlan& p, int tab
   p.off_buckets = take((size_t)windows * p.nb * 128);
   // the runs, and for buckets of many of them: chunk and bucket records, counters,
   // chunk sums
-  const size_t lists = (size_t)p.max_chunks * (sizeof(MergeChunk) + sizeof(MergeBig));
-  p.off_merge = take(std::max((size_t)2 * p.T1 * 4, lists));
+  p.off_merge = take((size_t)p.max_chunks * (sizeof(MergeChunk) + sizeof(MergeBig)));
   p.off_slots = take((size_t)2 * p.T1 * 128);
-  const int64_t share = p.T1 > 1 ? (2 * p.T1 + p.k2 - 1) / p.k2 : 1;
-  p.off_merge_counts = take((size_t)2 * share * 4);
-  p.off_merge_sums = take(std::max((size_t)2 * share * 128, (size_t)p.max_chunks * 128));
-  const int64_t chunks = (p.nb + ((int64_t)32 << p.red_l) - 1) >> (5 + p.red_l);
-  const int64_t red = windows * std::max<int64_t>({p.nb >> p.log_l, chunks, 1});
+  p.off_merge_counts = take(2 * 4);
+  p.off_merge_sums = take((size_t)p.max_chunks * 128);
+  // the first reduction level's pairs, the most of any level
+  const int64_t red = windows * ((p.nb + ((int64_t)32 << p.red_l) - 1) >> (5 + p.red_l));
   p.off_red_s0 = take((size_t)red * 128);
   p.off_red_u0 = take((size_t)red * 128);
   p.off_red_s1 = take((size_t)red * 128);
