@@ -1766,11 +1766,12 @@ static int make_plan(const int64_t* sizes, int count, int w, MsmPlan& p, int tab
   // pairs per bucket thread: the knob, else by size. A thread adds its pairs one
   // after another, so small MSMs want short chains and many threads; each thread
   // may leave two partial sums for the merge, so large ones want long
-  // chains. E / 2^19 rounded down to a power of two, within 8..64: measured on
-  // B200 (uniform scalars, default windows), 8 pairs against 64 take 2^10 points
-  // from 1.89 to 1.56 ms, 2^14 from 2.07 to 1.79, 2^16 from 2.36 to 2.14; from
-  // 2^19 points 16-32 pairs match 64 (skewed scalars gain 5-12 %), and 2^21 up
-  // keeps 64.
+  // chains. E / 2^19 rounded down to a power of two, within 8..64. Measured on
+  // B200 (one MSM, default windows), 8 / 16 / 32 / 64 pairs, uniform scalars:
+  // 2^10 points 0.34 / 0.37 / 0.44 / 0.59 ms, 2^14 0.49 / 0.52 / 0.53 / 0.65,
+  // 2^16 0.67 / 0.66 / 0.67 / 0.78, 2^18 1.44 / 1.35 / 1.32 / 1.41, 2^20 3.85 /
+  // 3.50 / 3.37 / 3.32, 2^22 13.4 / 12.0 / 11.4 / 11.1; skewed ones: 2^16 0.55 /
+  // 0.54 / 0.58 / 0.73, 2^20 1.59 / 1.50 / 1.48 / 1.57, 2^22 4.41 / 4.05 / 3.87 / 3.82.
   p.k1 = k1 > 0 ? k1 : tune_get("msm.pairs_per_thread");
   if (p.k1 < 8) {
     p.k1 = 8;
@@ -2074,7 +2075,7 @@ static int run_msm(const MsmJobs& J, const MsmPlan& p, char* ws, cudaStream_t s)
   // 5. finalize
   ProfSpan fin_span("msm_finalize", s);
   // with tables there is one window sum per job: nothing to combine
-  if (p.table || p.W == 1) {
+  if (p.table) {
     k_msm_finalize_one<<<(unsigned)p.count, 32, 0, s>>>(J, wsum);
   } else {
     k_msm_finalize<<<(unsigned)p.count, 32, 0, s>>>(J, wsum, p.W, p.w);
@@ -2353,9 +2354,9 @@ extern "C" {
 // All calls share the one array per device, so two calls whose work overlaps
 // on the GPU (different streams, or different host threads) corrupt each
 // other's results: callers must order them, for example on one stream.
-// Every buffer the pipeline reads is fully rewritten by the call itself (the
-// buckets are reset to the identity, every key and slot is written before it
-// is read), so a call never depends on what the previous one left behind.
+// Every buffer the pipeline reads is fully rewritten by the call itself (each
+// bucket by its one thread or by the merge, the empty ones with the identity;
+// every key and slot before it is read), so a call never depends on what the previous one left behind.
 
 namespace zkb {
 
